@@ -2,19 +2,30 @@
 // dealt into value slots by a monotone linear map of their offset from the
 // bucket's minimum, the slots are laid out by an exclusive scan of their
 // counts, the keys are dealt into their slots, and each slot that received
-// more than one key (a few keys at most) is put in order in place by the
-// thread that scanned it; the buffer is then the sorted bucket.
+// more than one key (a few keys at most) is put in order in place by one
+// thread; the buffer is then the sorted bucket.
 //
 // A bucket that reaches the leaf stage holds the keys between two adjacent
 // quantile splitters, so its values are close to evenly spread over
-// [min, max]: with as many slots as the class has keys, a slot holds about
-// one key and the whole sort costs a few shared-memory operations per key,
-// where a comparison network costs one compare-exchange per key for every
-// stage.  When the spread is uneven (a cluster, a run of repeated values, an
-// outlier that stretches the range) the slot counts show it before any key
-// moves: if the largest slot exceeds SLOT_MAX_RUN keys, or the ranking work
-// (the sum of squared slot counts) exceeds SLOT_SUMSQ per key, the bucket is
-// sorted by the bitonic + merge-path block sort instead (s512_blocksort.cuh).
+// [min, max]: with four slots per key of the class, four keys in five have a
+// slot of their own and the whole sort costs a few shared-memory operations
+// per key, where a comparison network costs one compare-exchange per key for
+// every stage.  When the spread is uneven (a cluster, a run of repeated
+// values, an outlier that stretches the range) the slot counts show it before
+// any key moves: if a slot holds more than SLOT_MAX keys, or some thread's
+// keys met more than SLOT_MEET others each on average, the bucket is sorted
+// by the bitonic + merge-path block sort instead (s512_blocksort.cuh).
+//
+// What bounds it: issue slots and shared-memory latency, not HBM, so the code
+// is laid out for few instructions per key.  Four 8-bit slot counters share a
+// word: one atomic gives a key its rank in its slot, and the scan leaves in
+// the same word the first key's place (14 bits) and the running counts of the
+// word's first three slots (6 bits each), so a key finds its place with one
+// more load.  Measured: the leaves of 2^28 uniform doubles 2.46 -> 1.99 ms
+// against one 32-bit counter per key, a second atomic to deal it and 64-bit
+// bounds; one array of 10007 uniform doubles, whose bit patterns crowd into
+// the top binade, 48 -> 15 us, because four slots per key keep it out of the
+// block sort.
 //
 // Equal keys are identical encoded words (see s512_common.cuh), so placing
 // ties in any order gives the same output.
@@ -24,8 +35,9 @@
 
 namespace s512 {
 
-constexpr uint32_t SLOT_MAX_RUN = 32;  // largest slot put in order by one thread
-constexpr uint32_t SLOT_SUMSQ = 4;     // in-slot ordering work (sum of squared counts) allowed per key
+constexpr uint32_t SLOT_MAX = 15;   // largest slot put in order by one thread (4 * 15 < 64: the
+                                    // running counts of a word fit their 6 bits)
+constexpr uint32_t SLOT_MEET = 3;   // a thread's keys may meet this many earlier keys each, on average
 
 // Monotone map from a key in [lo, hi] to a slot in [0, nslots): the offset
 // x - lo is cut to its 32 leading significant bits (shift sh), then either
@@ -37,7 +49,9 @@ struct SlotMap {
     K lo;
     uint32_t sh, mul, direct;
     __device__ __forceinline__ uint32_t operator()(K x) const {
-        const uint32_t d = (uint32_t)((x - lo) >> sh);
+        uint32_t d;
+        if constexpr (sizeof(K) == 8) d = (uint32_t)((x - lo) >> sh);
+        else d = (uint32_t)(x - lo);  // (32-bit offsets need no shift)
         return direct ? d : __umulhi(d, mul);
     }
 };
@@ -57,31 +71,68 @@ __device__ __forceinline__ SlotMap<K> make_slot_map(K lo, K hi, uint32_t nslots)
     return f;
 }
 
+// The slot map of a bucket: make_slot_map with the quotient taken in float,
+// rounded down far enough that the largest offset stays below nslots (the
+// 64-bit division of make_slot_map costs as much as seven keys of work).
+template <typename K>
+__device__ __forceinline__ SlotMap<K> make_slot_map_fast(K lo, K range, uint32_t nslots) {
+    SlotMap<K> f;
+    f.lo = lo;
+    int nb;
+    if constexpr (sizeof(K) == 8) nb = 64 - __clzll((long long)range);
+    else nb = 32 - __clz((int)range);
+    f.sh = nb > 32 ? (uint32_t)(nb - 32) : 0u;
+    const uint32_t dr = (uint32_t)(range >> f.sh);
+    f.direct = dr < nslots ? 1u : 0u;
+    // relative error of the conversion, the divide and the product: under
+    // 2^-21; the factor takes off 2^-20
+    const float q = __fdividef((float)nslots * 4294967296.0f, (float)dr + 1.0f) * (1.0f - 1.0f / 1048576.0f);
+    f.mul = f.direct ? 0u : (uint32_t)q;
+    return f;
+}
+
 // Per-warp partials of the block reductions.
 template <typename K>
 struct SlotRed {
     K wlo[32], whi[32];
-    uint32_t wtot[32], wmax[32], wsq[32];
+    uint32_t hlo[32], hhi[32];
+    uint32_t wtot[32];
 };
 
 // Shared memory of block_slot_sort for a block of THREADS x IPT keys: the
-// key buffer (padded for the block sort when that runs inline, INLINE) and
-// the counters.
+// key buffer (padded for the block sort when that runs inline, INLINE), one
+// word of four slot counters per key, and the list of the slots that received
+// several keys (at most half as many as keys).
 template <typename K, int THREADS, int IPT, bool INLINE = true>
 struct SlotSmem {
     static constexpr uint32_t S = (uint32_t)THREADS * IPT;
     static constexpr size_t keys_bytes = ((size_t)(INLINE ? padded_len(S) : S) * sizeof(K) + 15) & ~(size_t)15;
     static constexpr size_t ctr_bytes = (size_t)S * sizeof(uint32_t);
-    static constexpr size_t bytes = keys_bytes + ctr_bytes;
+    static constexpr size_t list_bytes = (size_t)S;
+    static constexpr size_t bytes = keys_bytes + ctr_bytes + list_bytes;
 };
+
+// Byte offset of a counter word in shared memory.  A thread scans IPT
+// consecutive words as 16-byte quads; exchanging quads within a thread's
+// group keeps the eight lanes of a quad access on different banks (their
+// stride would otherwise put them four or two to a bank; at IPT 12 the stride
+// does it by itself).  The exchange is its own inverse.
+template <int IPT>
+__device__ __forceinline__ uint32_t ctr_swizzle(uint32_t a) {
+    constexpr uint32_t Q = IPT / 4;
+    if constexpr (Q == 2 || Q == 4) return a ^ ((a >> 3) & ((Q - 1) << 4));
+    else return a;
+}
 
 // Sort the c <= THREADS*IPT keys held striped in key[] (element
 // r*THREADS + tid in key[r]; entries past c are ignored) into store(0..c).
 // `smem` holds SlotSmem<K,THREADS,IPT>::bytes; `red` is the block's reduction
 // scratch.  refill() is called exactly once, as soon as key[] is no longer
 // needed, so that the caller can start loading the next bucket into it while
-// this one is ranked and written.  Every thread of the block must call it; it
-// ends with a barrier, so the caller may reuse the shared memory right after.
+// this one is ranked and written.  Every thread of the block must call it.
+// The key buffer may still be read by other threads when it returns; another
+// call may follow directly (it does not write that buffer before its own
+// barriers), anything else needs a barrier first.
 // Returns true when the bucket took the distribution-counting path.
 //
 // An uneven bucket is sorted here by the block sort when INLINE_FALLBACK is
@@ -92,146 +143,205 @@ template <typename K, int THREADS, int IPT, bool INLINE_FALLBACK, typename Store
 __device__ bool block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refill refill, Uneven uneven,
                                 unsigned char* smem, SlotRed<K>& red) {
     constexpr uint32_t S = (uint32_t)THREADS * IPT;
+    constexpr uint32_t NSLOTS = 4 * S;
     constexpr int NW = THREADS / 32;
-    static_assert(IPT % 4 == 0 && IPT <= 32, "counters are read four at a time, slot bits in one word");
+    static_assert(IPT % 4 == 0 && IPT <= 16, "counter words are read four at a time");
+    static_assert(S <= 16384, "a place is 14 bits, a counter's byte offset 16");
     using SM = SlotSmem<K, THREADS, IPT, INLINE_FALLBACK>;
     K* s = reinterpret_cast<K*>(smem);
-    uint32_t* ctr = reinterpret_cast<uint32_t*>(smem + SM::keys_bytes);
+    unsigned char* ctr = smem + SM::keys_bytes;
+    uint16_t* list = reinterpret_cast<uint16_t*>(smem + SM::keys_bytes + SM::ctr_bytes);
     const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
 
-    // 1. bounds of the bucket; counters zeroed
-    K lo = KeyMax<K>::value, hi = K(0);
+    // 1. bounds of the bucket; counters zeroed.  Of 64-bit keys only the high
+    // words are compared: unless they span very few values, the bounds need
+    // no more precision.
+    uint32_t hmin = 0xFFFFFFFFu, hmax = 0u;
 #pragma unroll
     for (int r = 0; r < IPT; ++r) {
         if ((uint32_t)r * THREADS + tid < c) {
-            lo = kmin(lo, key[r]);
-            hi = kmax(hi, key[r]);
+            const uint32_t h = sizeof(K) == 8 ? (uint32_t)((uint64_t)key[r] >> 32) : (uint32_t)key[r];
+            hmin = min(hmin, h);
+            hmax = max(hmax, h);
         }
     }
 #pragma unroll
     for (int r = 0; r < IPT; r += 4)
-        *reinterpret_cast<uint4*>(&ctr[tid * IPT + r]) = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        lo = kmin(lo, shfl_xor(lo, d));
-        hi = kmax(hi, shfl_xor(hi, d));
-    }
+        *reinterpret_cast<uint4*>(ctr + (size_t)tid * IPT * 4 + r * 4) = make_uint4(0u, 0u, 0u, 0u);
+    hmin = __reduce_min_sync(0xFFFFFFFFu, hmin);
+    hmax = __reduce_max_sync(0xFFFFFFFFu, hmax);
     if (lane == 0) {
-        red.wlo[warp] = lo;
-        red.whi[warp] = hi;
+        red.hlo[warp] = hmin;
+        red.hhi[warp] = hmax;
     }
     __syncthreads();
-    lo = lane < (unsigned)NW ? red.wlo[lane] : KeyMax<K>::value;
-    hi = lane < (unsigned)NW ? red.whi[lane] : K(0);
+    hmin = __reduce_min_sync(0xFFFFFFFFu, lane < (unsigned)NW ? red.hlo[lane] : 0xFFFFFFFFu);
+    hmax = __reduce_max_sync(0xFFFFFFFFu, lane < (unsigned)NW ? red.hhi[lane] : 0u);
+    K lo, range;
+    if constexpr (sizeof(K) == 8) {
+        lo = (uint64_t)hmin << 32;
+        range = ((uint64_t)(hmax - hmin) << 32) | 0xFFFFFFFFull;
+        if (hmax - hmin < 4096u) {  // few high words: exact bounds
+            K mn = KeyMax<K>::value, mx = K(0);
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        lo = kmin(lo, shfl_xor(lo, d));
-        hi = kmax(hi, shfl_xor(hi, d));
+            for (int r = 0; r < IPT; ++r) {
+                if ((uint32_t)r * THREADS + tid < c) {
+                    mn = kmin(mn, key[r]);
+                    mx = kmax(mx, key[r]);
+                }
+            }
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) {
+                mn = kmin(mn, shfl_xor(mn, d));
+                mx = kmax(mx, shfl_xor(mx, d));
+            }
+            if (lane == 0) {
+                red.wlo[warp] = mn;
+                red.whi[warp] = mx;
+            }
+            __syncthreads();
+            mn = lane < (unsigned)NW ? red.wlo[lane] : KeyMax<K>::value;
+            mx = lane < (unsigned)NW ? red.whi[lane] : K(0);
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) {
+                mn = kmin(mn, shfl_xor(mn, d));
+                mx = kmax(mx, shfl_xor(mx, d));
+            }
+            lo = mn;
+            range = mx - mn;
+        }
+    } else {
+        lo = hmin;
+        range = hmax - hmin;
     }
 
-    if (lo == hi) {  // every key equal: already in order
+    if (range == 0) {  // every key equal: already in order
 #pragma unroll
         for (int r = 0; r < IPT; ++r) {
             const uint32_t i = (uint32_t)r * THREADS + tid;
             if (i < c) store(i, key[r]);
         }
         refill();
-        __syncthreads();
+        __syncthreads();  // (the counters and bounds are rewritten by the next call)
         return true;
     }
 
-    // 2. slot counts
-    const SlotMap<K> f = make_slot_map<K>(lo, hi, S);
+    // 2. slot counts: a key's rank in its slot is its counter's byte before
+    // the key's own increment.  (A byte that passes 255 carries into its
+    // neighbour, but then a key has seen the rank SLOT_MAX and the counts are
+    // not used.)
+    const SlotMap<K> f = make_slot_map_fast<K>(lo, range, NSLOTS);
+    uint32_t pr[IPT];  // counter byte offset | slot within the word | rank << 16
+    uint32_t rmax = 0, rsum = 0, nmulti = 0;
 #pragma unroll
     for (int r = 0; r < IPT; ++r) {
-        if ((uint32_t)r * THREADS + tid < c) atomicAdd(&ctr[f(key[r])], 1u);
+        pr[r] = 0;
+        if ((uint32_t)r * THREADS + tid < c) {
+            const uint32_t slot = f(key[r]);
+            const uint32_t a = ctr_swizzle<IPT>(slot & ~3u);
+            const uint32_t k8 = slot << 3;  // (shifts take it modulo 32)
+            const uint32_t old = atomicAdd(reinterpret_cast<uint32_t*>(ctr + a), __funnelshift_l(0u, 1u, k8));
+            const uint32_t rank = __funnelshift_r(old, 0u, k8) & 0xFFu;
+            pr[r] = (a | (slot & 3u)) + (rank << 16);
+            rmax = max(rmax, rank);
+            rsum += rank;
+            nmulti += rank == 1u ? 1u : 0u;
+        }
     }
-    __syncthreads();
-
-    // 3. exclusive scan of the counts (IPT consecutive counters per thread)
-    //    with the largest count and the sum of squared counts; one barrier:
-    //    every warp scans the per-warp totals itself
-    uint32_t sum = 0, mx = 0, sq = 0;
-#pragma unroll
-    for (int r = 0; r < IPT; r += 4) {
-        const uint4 q = *reinterpret_cast<const uint4*>(&ctr[tid * IPT + r]);
-        sum += q.x + q.y + q.z + q.w;
-        mx = max(max(mx, max(q.x, q.y)), max(q.z, q.w));
-        sq += q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
-    }
-    uint32_t inc = sum;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, inc, d);
-        if (lane >= (unsigned)d) inc += o;
-    }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, d));
-        sq += __shfl_xor_sync(0xFFFFFFFFu, sq, d);
-    }
-    if (lane == 31) red.wtot[warp] = inc;
-    if (lane == 0) {
-        red.wmax[warp] = mx;
-        red.wsq[warp] = sq;
-    }
-    __syncthreads();
-    uint32_t before = (lane < warp) ? red.wtot[lane] : 0u;
-    mx = lane < (unsigned)NW ? red.wmax[lane] : 0u;
-    sq = lane < (unsigned)NW ? red.wsq[lane] : 0u;
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        before += __shfl_xor_sync(0xFFFFFFFFu, before, d);
-        mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, d));
-        sq += __shfl_xor_sync(0xFFFFFFFFu, sq, d);
-    }
-    const bool even = mx <= SLOT_MAX_RUN && sq <= SLOT_SUMSQ * c;
+    const bool even = !__syncthreads_or(rmax >= SLOT_MAX || rsum > SLOT_MEET * IPT);
 
     if (even) {
-        // counts -> slot starts (the counters are read again rather than kept
-        // in registers across the barrier)
-        uint32_t run = before + inc - sum;
-        uint32_t mbits = 0;  // bit r: slot tid*IPT + r holds more than one key
+        // 3. exclusive scan of the counts (IPT consecutive words per thread)
+        // and, in the high half, of the slots with several keys (each counted
+        // by the thread whose key came second)
+        uint32_t v = nmulti << 16;
+        unsigned char* own = ctr + (size_t)tid * IPT * 4;
+        auto quad = [&](int j) {
+            return reinterpret_cast<uint4*>(ctr + ctr_swizzle<IPT>((uint32_t)(own - ctr) + (uint32_t)j * 16));
+        };
 #pragma unroll
-        for (int r = 0; r < IPT; r += 4) {
-            uint4 q = *reinterpret_cast<const uint4*>(&ctr[tid * IPT + r]);
-            mbits |= ((q.x > 1u) ? 1u : 0u) << r | ((q.y > 1u) ? 1u : 0u) << (r + 1) |
-                     ((q.z > 1u) ? 1u : 0u) << (r + 2) | ((q.w > 1u) ? 1u : 0u) << (r + 3);
-            const uint32_t s0 = run, s1 = s0 + q.x, s2 = s1 + q.y, s3 = s2 + q.z;
-            run = s3 + q.w;
-            q = make_uint4(s0, s1, s2, s3);
-            *reinterpret_cast<uint4*>(&ctr[tid * IPT + r]) = q;
+        for (int j = 0; j < IPT / 4; ++j) {
+            const uint4 q = *quad(j);
+            v += (q.x * 0x01010101u) >> 24;
+            v += (q.y * 0x01010101u) >> 24;
+            v += (q.z * 0x01010101u) >> 24;
+            v += (q.w * 0x01010101u) >> 24;
+        }
+        uint32_t inc = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, inc, d);
+            if (lane >= (unsigned)d) inc += o;
+        }
+        if (lane == 31) red.wtot[warp] = inc;
+        __syncthreads();
+        const uint32_t wt = lane < (unsigned)NW ? red.wtot[lane] : 0u;
+        const uint32_t before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? wt : 0u);
+        const uint32_t nlist = __reduce_add_sync(0xFFFFFFFFu, wt) >> 16;
+        uint32_t run = before + inc - v;
+        uint32_t li = run >> 16;
+        run &= 0xFFFFu;
+        // the word's first place and its slots' running counts (the counters
+        // are read again rather than kept in registers across the barrier)
+#pragma unroll
+        for (int j = 0; j < IPT / 4; ++j) {
+            uint4* qp = quad(j);
+            uint4 q = *qp;
+            auto start = [&](uint32_t w) {
+                const uint32_t m = w * 0x01010101u;  // byte k: keys in slots 0..k of the word
+                const uint32_t p = (run << 18) | ((m >> 4) & 0x3F000u) | ((m >> 2) & 0xFC0u) | (m & 0x3Fu);
+                run += m >> 24;
+                return p;
+            };
+            q.x = start(q.x);
+            q.y = start(q.y);
+            q.z = start(q.z);
+            q.w = start(q.w);
+            *qp = q;
         }
         __syncthreads();
-        // 4. deal the keys into their slots; afterwards ctr[j] is the end of slot j
+        // 4. deal the keys into their places, and list the slots of several
 #pragma unroll
         for (int r = 0; r < IPT; ++r) {
-            if ((uint32_t)r * THREADS + tid < c) s[atomicAdd(&ctr[f(key[r])], 1u)] = key[r];
+            if ((uint32_t)r * THREADS + tid < c) {
+                const uint32_t w = *reinterpret_cast<const uint32_t*>(ctr + (pr[r] & 0xFFFCu));
+                const uint32_t rank = pr[r] >> 16;
+                s[(w >> 18) + (((w << 6) >> ((pr[r] & 3u) * 6u)) & 63u) + rank] = key[r];
+                if (rank == 1u) list[li++] = (uint16_t)pr[r];
+            }
         }
         refill();
         __syncthreads();
-        // 5. the keys of a slot of several are in dealing order: the thread
-        //    that scanned the slot puts them in key order, in place
-        for (uint32_t bits = mbits; bits; bits &= bits - 1) {
-            const uint32_t j = tid * IPT + (uint32_t)(__ffs(bits) - 1);
-            const uint32_t a = j ? ctr[j - 1] : 0u;
-            const uint32_t e = ctr[j];
-            if (e - a == 2) {
-                const K x0 = s[a], x1 = s[a + 1];
+        // 5. the keys of a slot of several are in dealing order: one thread
+        // puts them in key order, in place
+        for (uint32_t q = tid; q < nlist; q += THREADS) {
+            const uint32_t e = list[q];
+            const uint32_t pa = e & 0xFFFCu, k = e & 3u;
+            const uint32_t w = *reinterpret_cast<const uint32_t*>(ctr + pa);
+            const uint32_t na = ctr_swizzle<IPT>(pa) + 4u;  // the next word's logical offset
+            const uint32_t wn =
+                na < S * 4 ? *reinterpret_cast<const uint32_t*>(ctr + ctr_swizzle<IPT>(na)) : c << 18;
+            const uint32_t w6 = w << 6;
+            const uint32_t f0 = (w6 >> (k * 6u)) & 63u;
+            const uint32_t f1 =  // (places are 14 bits: the difference is taken modulo 2^14)
+                k == 3u ? ((wn >> 18) - (w >> 18)) & 0x3FFFu : (w6 >> (k * 6u + 6u)) & 63u;
+            const uint32_t a0 = (w >> 18) + f0, n = f1 - f0;
+            if (n == 2) {
+                const K x0 = s[a0], x1 = s[a0 + 1];
                 if (x1 < x0) {
-                    s[a] = x1;
-                    s[a + 1] = x0;
+                    s[a0] = x1;
+                    s[a0 + 1] = x0;
                 }
             } else {
-                for (uint32_t q = a + 1; q < e; ++q) {
-                    const K x = s[q];
-                    uint32_t k = q;
-                    for (; k > a; --k) {
-                        const K y = s[k - 1];
+                for (uint32_t i = a0 + 1; i < a0 + n; ++i) {
+                    const K x = s[i];
+                    uint32_t t = i;
+                    for (; t > a0; --t) {
+                        const K y = s[t - 1];
                         if (!(x < y)) break;
-                        s[k] = y;
+                        s[t] = y;
                     }
-                    s[k] = x;
+                    s[t] = x;
                 }
             }
         }
@@ -248,11 +358,11 @@ __device__ bool block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refill r
         block_merge_sort<K, THREADS, IPT>(s, c);
         for (uint32_t i = tid; i < c; i += THREADS) store(i, s[pidx(i)]);
         refill();  // (after the merge, which needs the registers)
+        __syncthreads();
     } else {
         if (tid == 0) uneven();
         refill();
     }
-    __syncthreads();
     return even;
 }
 
