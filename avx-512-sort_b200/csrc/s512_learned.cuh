@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(LR_THREADS) learned_root_kernel(const K* __res
     __syncthreads();
     bool fit = sd.count >= LR_MIN_KEYS;
     bool searches = false;
-    if (fit) {
+    if (fit && !plain[sgi].direct) {  // (a direct table never searches, and its sample is not sorted)
         const SplitSet<K>& ps = plain[sgi];
         const SlotMap<K> fmap = ps.slot_map;
         uint32_t mine = 0;
@@ -350,6 +350,8 @@ __global__ void __launch_bounds__(LR_THREADS) learned_root_kernel(const K* __res
         __syncthreads();
         searches = (float)search_s > LR_TABLE_SEARCH_FRAC * (float)m;
         fit = searches || force;
+    } else {
+        fit = false;
     }
     if (!fit) {  // the split set routes it
         if (tid == 0) {

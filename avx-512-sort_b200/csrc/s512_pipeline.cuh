@@ -143,7 +143,7 @@ static inline int wait_feed(const HostFeed* feed, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// One partition level: sample -> sort sample -> splitters -> partition -> plan.
+// One partition level: sorted sample and splitters -> partition -> plan.
 template <typename K, typename InCodec>
 struct Level {
     InCodec in;
@@ -185,21 +185,20 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
     S512_CUDA_TRY(cudaMemsetAsync(ctl, 0, sizeof(LevelCtl), st));
     S512_CUDA_TRY(cudaMemsetAsync(counts, 0, (size_t)nsegs * NB * sizeof(uint64_t), st));
     const uint64_t seed = config().seed + 0x9E3779B97F4A7C15ull * (uint64_t)(level + 1);
-    if (feed)  // the caller's host arrays, read where they are
-        sample_kernel<InCodec><<<nsegs, 256, 0, st>>>(L.in.rebased(feed->mapped), L.segs, nsegs, samples, seed, KB);
-    else
-        sample_kernel<InCodec><<<nsegs, 256, 0, st>>>(L.in, L.segs, nsegs, samples, seed, KB);
-    S512_LAUNCH_CHECK();
     {
-        auto fn = sample_sort_kernel<K>;
-        const size_t smem = SlotSmem<K, 1024, SAMPLE_N / 1024>::bytes;
-        S512_CUDA_TRY(C.prepare((const void*)fn, smem));
-        fn<<<nsegs, 1024, smem, st>>>(samples, L.segs, nsegs, KB);
+        // enough blocks per segment to fill the chip (a fed level reads the
+        // caller's host arrays where they are)
+        uint32_t parts = 2368u / nsegs;
+        parts = parts < 1 ? 1u : parts > SAMPLE_N / 256 ? SAMPLE_N / 256 : parts;
+        sample_kernel<InCodec><<<nsegs * parts, 256, 0, st>>>(feed ? L.in.rebased(feed->mapped) : L.in, L.segs, parts,
+                                                              samples, seed, KB);
+        S512_LAUNCH_CHECK();
+        auto fn = split_kernel<K>;
+        S512_CUDA_TRY(C.prepare((const void*)fn, split_smem<K>()));
+        fn<<<nsegs, SAMPLE_THREADS, split_smem<K>(), st>>>(samples, L.segs, splits, KB, learned ? 1 : 0);
         S512_LAUNCH_CHECK();
     }
-    splitter_kernel<K><<<nsegs, NB, 0, st>>>(samples, L.segs, nsegs, splits, KB);
-    S512_LAUNCH_CHECK();
-    S.kernel_launches += 3;
+    S.kernel_launches += 2;
     int tfit0 = -1;
     if (learned) {
         // the model is fitted to the same sorted sample; the split set above

@@ -91,6 +91,8 @@ __device__ __forceinline__ SlotMap<K> make_slot_map_fast(K lo, K range, uint32_t
     return f;
 }
 
+enum SlotPath { SLOT_EQUAL, SLOT_EVEN, SLOT_UNEVEN };
+
 // Per-warp partials of the block reductions.
 template <typename K>
 struct SlotRed {
@@ -124,38 +126,14 @@ __device__ __forceinline__ uint32_t ctr_swizzle(uint32_t a) {
     else return a;
 }
 
-// Sort the c <= THREADS*IPT keys held striped in key[] (element
-// r*THREADS + tid in key[r]; entries past c are ignored) into store(0..c).
-// `smem` holds SlotSmem<K,THREADS,IPT>::bytes; `red` is the block's reduction
-// scratch.  refill() is called exactly once, as soon as key[] is no longer
-// needed, so that the caller can start loading the next bucket into it while
-// this one is ranked and written.  Every thread of the block must call it.
-// The key buffer may still be read by other threads when it returns; another
-// call may follow directly (it does not write that buffer before its own
-// barriers), anything else needs a barrier first.
-// Returns true when the bucket took the distribution-counting path.
-//
-// An uneven bucket is sorted here by the block sort when INLINE_FALLBACK is
-// set; otherwise thread 0 calls uneven() (which hands the bucket to a
-// separate launch) and nothing is written.  Keeping the block sort out of
-// the kernel keeps the slot path's register budget for the keys.
-template <typename K, int THREADS, int IPT, bool INLINE_FALLBACK, typename Store, typename Refill, typename Uneven>
-__device__ bool block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refill refill, Uneven uneven,
-                                unsigned char* smem, SlotRed<K>& red) {
-    constexpr uint32_t S = (uint32_t)THREADS * IPT;
-    constexpr uint32_t NSLOTS = 4 * S;
+// Bounds of the c keys held striped in key[]: lo <= every key <= lo + range.
+// Of 64-bit keys only the high words are compared: unless they span very few
+// values, the bounds need no more precision (range == 0 is always exact).
+// Every thread of the block calls it; it has a barrier.
+template <typename K, int THREADS, int IPT>
+__device__ __forceinline__ void block_bounds(const K (&key)[IPT], uint32_t c, SlotRed<K>& red, K& lo, K& range) {
     constexpr int NW = THREADS / 32;
-    static_assert(IPT % 4 == 0 && IPT <= 16, "counter words are read four at a time");
-    static_assert(S <= 16384, "a place is 14 bits, a counter's byte offset 16");
-    using SM = SlotSmem<K, THREADS, IPT, INLINE_FALLBACK>;
-    K* s = reinterpret_cast<K*>(smem);
-    unsigned char* ctr = smem + SM::keys_bytes;
-    uint16_t* list = reinterpret_cast<uint16_t*>(smem + SM::keys_bytes + SM::ctr_bytes);
     const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-
-    // 1. bounds of the bucket; counters zeroed.  Of 64-bit keys only the high
-    // words are compared: unless they span very few values, the bounds need
-    // no more precision.
     uint32_t hmin = 0xFFFFFFFFu, hmax = 0u;
 #pragma unroll
     for (int r = 0; r < IPT; ++r) {
@@ -165,9 +143,6 @@ __device__ bool block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refill r
             hmax = max(hmax, h);
         }
     }
-#pragma unroll
-    for (int r = 0; r < IPT; r += 4)
-        *reinterpret_cast<uint4*>(ctr + (size_t)tid * IPT * 4 + r * 4) = make_uint4(0u, 0u, 0u, 0u);
     hmin = __reduce_min_sync(0xFFFFFFFFu, hmin);
     hmax = __reduce_max_sync(0xFFFFFFFFu, hmax);
     if (lane == 0) {
@@ -177,7 +152,6 @@ __device__ bool block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refill r
     __syncthreads();
     hmin = __reduce_min_sync(0xFFFFFFFFu, lane < (unsigned)NW ? red.hlo[lane] : 0xFFFFFFFFu);
     hmax = __reduce_max_sync(0xFFFFFFFFu, lane < (unsigned)NW ? red.hhi[lane] : 0u);
-    K lo, range;
     if constexpr (sizeof(K) == 8) {
         lo = (uint64_t)hmin << 32;
         range = ((uint64_t)(hmax - hmin) << 32) | 0xFFFFFFFFull;
@@ -214,6 +188,45 @@ __device__ bool block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refill r
         lo = hmin;
         range = hmax - hmin;
     }
+}
+
+// Sort the c <= THREADS*IPT keys held striped in key[] (element
+// r*THREADS + tid in key[r]; entries past c are ignored) into store(0..c).
+// `smem` holds SlotSmem<K,THREADS,IPT>::bytes; `red` is the block's reduction
+// scratch.  refill() is called exactly once, as soon as key[] is no longer
+// needed, so that the caller can start loading the next bucket into it while
+// this one is ranked and written.  Every thread of the block must call it.
+// The key buffer may still be read by other threads when it returns; another
+// call may follow directly (it does not write that buffer before its own
+// barriers), anything else needs a barrier first.
+// Returns how the bucket was sorted, hence where its sorted keys are left in
+// the key buffer: in order (SLOT_EVEN), in the block sort's padded layout
+// (SLOT_UNEVEN, with INLINE_FALLBACK), or nowhere (SLOT_EQUAL).
+//
+// An uneven bucket is sorted here by the block sort when INLINE_FALLBACK is
+// set; otherwise thread 0 calls uneven() (which hands the bucket to a
+// separate launch) and nothing is written.  Keeping the block sort out of
+// the kernel keeps the slot path's register budget for the keys.
+template <typename K, int THREADS, int IPT, bool INLINE_FALLBACK, typename Store, typename Refill, typename Uneven>
+__device__ SlotPath block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refill refill, Uneven uneven,
+                                unsigned char* smem, SlotRed<K>& red) {
+    constexpr uint32_t S = (uint32_t)THREADS * IPT;
+    constexpr uint32_t NSLOTS = 4 * S;
+    constexpr int NW = THREADS / 32;
+    static_assert(IPT % 4 == 0 && IPT <= 16, "counter words are read four at a time");
+    static_assert(S <= 16384, "a place is 14 bits, a counter's byte offset 16");
+    using SM = SlotSmem<K, THREADS, IPT, INLINE_FALLBACK>;
+    K* s = reinterpret_cast<K*>(smem);
+    unsigned char* ctr = smem + SM::keys_bytes;
+    uint16_t* list = reinterpret_cast<uint16_t*>(smem + SM::keys_bytes + SM::ctr_bytes);
+    const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+
+    // 1. counters zeroed; bounds of the bucket
+#pragma unroll
+    for (int r = 0; r < IPT; r += 4)
+        *reinterpret_cast<uint4*>(ctr + (size_t)tid * IPT * 4 + r * 4) = make_uint4(0u, 0u, 0u, 0u);
+    K lo, range;
+    block_bounds<K, THREADS, IPT>(key, c, red, lo, range);
 
     if (range == 0) {  // every key equal: already in order
 #pragma unroll
@@ -223,7 +236,7 @@ __device__ bool block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refill r
         }
         refill();
         __syncthreads();  // (the counters and bounds are rewritten by the next call)
-        return true;
+        return SLOT_EQUAL;
     }
 
     // 2. slot counts: a key's rank in its slot is its counter's byte before
@@ -363,7 +376,7 @@ __device__ bool block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refill r
         if (tid == 0) uneven();
         refill();
     }
-    return even;
+    return even ? SLOT_EVEN : SLOT_UNEVEN;
 }
 
 }  // namespace s512

@@ -37,6 +37,7 @@ constexpr int NB = 256;            // buckets per segment per pass (max)
 constexpr int SAMPLE_N = 16384;    // keys sampled per segment
 constexpr int COPY_CHUNK = 16384;  // equality buckets are copied in chunks of this size
 constexpr int SPLIT_SLOTS = 4096;  // value slots of the splitter lookup table
+constexpr int DIRECT_SLOTS = 16384;  // value slots of the direct table (segments split at slot boundaries)
 
 // A segment to partition at some level.
 struct SegDesc {
@@ -46,6 +47,42 @@ struct SegDesc {
     uint64_t out_base;   // start of the segment's bucket regions in the level's output
     uint32_t tile_start; // first global tile index of the segment
     uint32_t ntiles;
+};
+
+// Slot of a key in the direct table: its offset from lo, cut to 32 bits, times
+// a fixed-point factor.  fast() is right for keys in [lo, lo + range] and sets
+// `out` for any below lo or too far above; slot() is right for all (keys
+// outside clamp to the ends).  Both stay below DIRECT_SLOTS for any key.
+template <typename K>
+struct DirectMap {
+    K lo;
+    uint32_t sh, mul;
+    uint32_t dmax;   // cut offset of the upper bound
+    uint32_t hmax;   // 64-bit keys: its high word
+    __device__ __forceinline__ uint32_t cut(K d) const {
+        if constexpr (sizeof(K) == 8)
+            return min(__funnelshift_rc((uint32_t)d, (uint32_t)((uint64_t)d >> 32), sh), dmax);  // sh <= 32
+        else
+            return min((uint32_t)d, dmax);
+    }
+    __device__ __forceinline__ bool outside(K d) const {
+        if constexpr (sizeof(K) == 8) return (uint32_t)((uint64_t)d >> 32) > hmax;
+        else return (uint32_t)d > dmax;
+    }
+    __device__ __forceinline__ uint32_t fast(K x, bool& out) const {
+        const K d = x - lo;
+        out |= outside(d);
+        return __umulhi(cut(d), mul);
+    }
+    __device__ __forceinline__ uint32_t slot(K x) const {
+        const K d = x < lo ? K(0) : x - lo;
+        return __umulhi(outside(d) ? dmax : cut(d), mul);
+    }
+    // the smallest key of slot s or above (s at most slot(lo + range), not 0)
+    __device__ __forceinline__ K first_key(uint32_t s) const {
+        const uint32_t d = (uint32_t)((((uint64_t)s << 32) + mul - 1) / mul);
+        return lo + ((K)d << sh);
+    }
 };
 
 // Splitters of one segment and the layout of its bucket regions.
@@ -73,6 +110,12 @@ struct SplitSet {
     SlotMap<K> slot_map;
     K slot_hi;
     alignas(16) uint16_t slot_tab[SPLIT_SLOTS + 8];
+    // A segment whose sample spreads over many slots is split at slot
+    // boundaries (direct): a key's bucket is then dir_tab[dir_map(key)], with
+    // no splitter left to compare (uniq holds the same boundaries as keys).
+    uint32_t direct;
+    DirectMap<K> dir_map;
+    alignas(16) uint8_t dir_tab[DIRECT_SLOTS];
 };
 
 // A bucket that a leaf kernel sorts (or copies) into its final place.
@@ -151,197 +194,350 @@ struct LevelCtl {
 };
 
 // ===========================================================================
-// 1. Sampling: SAMPLE_N keys per segment at hashed positions (with replacement)
+// 1. Sampling: per segment, up to SAMPLE_N keys at hashed positions (with
+// replacement), sorted, and the splitters and bucket regions they give
 
-template <typename Codec>
-__global__ void sample_kernel(Codec in, const SegDesc* __restrict__ segs, uint32_t nsegs,
-                              typename Codec::Key* __restrict__ samples, uint64_t seed, int key_bytes) {
-    const uint32_t s = blockIdx.x;
-    if (s >= nsegs) return;
-    const SegDesc sd = segs[s];
-    const uint32_t m = sample_size(target_buckets(key_bytes, sd.count));
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-        const uint64_t h = mix64(seed ^ ((uint64_t)s << 32) ^ (uint64_t)i);
-        const uint64_t pos = __umul64hi(h, sd.count);
-        samples[(size_t)s * SAMPLE_N + i] = in.load(sd.in_off + pos);
-    }
-}
-
-// 2. Sorting the samples: one block of 1024 threads per segment.
-template <typename K>
-__global__ void __launch_bounds__(1024) sample_sort_kernel(K* __restrict__ samples, const SegDesc* __restrict__ segs,
-                                                           uint32_t nsegs, int key_bytes) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ SlotRed<K> red;
-    constexpr int IPT = SAMPLE_N / 1024;
-    const uint32_t m = sample_size(target_buckets(key_bytes, segs[blockIdx.x].count));
-    K* p = samples + (size_t)blockIdx.x * SAMPLE_N;
-    K key[IPT];
-#pragma unroll
-    for (int r = 0; r < IPT; ++r) {
-        const uint32_t i = (uint32_t)r * 1024 + threadIdx.x;
-        if (i < m) key[r] = p[i];
-    }
-    // samples are spread like the segment's keys: distribution counting,
-    // with the block sort for skewed samples (s512_slotsort.cuh)
-    block_slot_sort<K, 1024, IPT, true>(
-        key, m, [&](uint32_t i, K x) { p[i] = x; }, [] {}, [] {}, smem_raw, red);
-}
-
-// 3. Splitters and bucket regions: one block of 256 threads per segment.
-template <typename K>
-__device__ __forceinline__ uint32_t lower_bound_dev(const K* a, uint32_t n, K v) {
+template <typename F>
+__device__ __forceinline__ uint32_t first_index(uint32_t n, F past) {  // first i in [0, n) with past(i), else n
     uint32_t lo = 0, hi = n;
     while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (a[mid] < v) lo = mid + 1; else hi = mid;
-    }
-    return lo;
-}
-template <typename K>
-__device__ __forceinline__ uint32_t upper_bound_dev(const K* a, uint32_t n, K v) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (!(v < a[mid])) lo = mid + 1; else hi = mid;
+        const uint32_t mid = (lo + hi) >> 1;
+        if (past(mid)) hi = mid; else lo = mid + 1;
     }
     return lo;
 }
 
+// Scratch of make_splitters.
 template <typename K>
-__global__ void __launch_bounds__(256) splitter_kernel(const K* __restrict__ samples, const SegDesc* __restrict__ segs,
-                                                       uint32_t nsegs, SplitSet<K>* __restrict__ splits,
-                                                       int key_bytes) {
-    const uint32_t s = blockIdx.x;
-    if (s >= nsegs) return;
-    __shared__ K cand[NB];
-    __shared__ K uniq[NB];
-    __shared__ uint32_t eqf[NB];
-    __shared__ uint32_t wtot[8];
-    __shared__ uint32_t total_u, total_eq;
-    __shared__ uint64_t cap_s[NB];
-    __shared__ uint64_t wtot64[8];
-    __shared__ uint64_t cap_total;
+struct SplitScratch {
+    K cand[NB], uniq[NB];
+    uint64_t cap[NB];
+    uint64_t wtot64[NB / 32];
+    uint32_t eqf[NB], sk[NB];
+    uint32_t wtot[NB / 32];
+    uint32_t beq[NB / 32];
+    uint32_t total_u, total_eq;
+};
 
-    const K* smp = samples + (size_t)s * SAMPLE_N;
-    const SegDesc sd = segs[s];
-    SplitSet<K>* out = splits + s;
+// Region capacity of a bucket that holds cnt of the m samples of a segment of
+// `count` keys (scale = count / m): 6 sigma above its expected size.
+__device__ __forceinline__ uint64_t bucket_cap(uint32_t cnt, double scale, uint64_t count) {
+    const float v = (float)cnt + 6.0f * sqrtf((float)cnt + 1.0f) + 16.0f;
+    uint64_t cap = (uint64_t)((double)v * scale) + 1;
+    if (cap > count) cap = count;
+    return (cap + 15) & ~15ull;
+}
+
+// Region offsets, the splitters and their search tree, and the equality masks
+// from w.cap, w.uniq and w.beq (complete: a barrier behind them).
+template <typename K>
+__device__ void write_layout(SplitSet<K>* out, SplitScratch<K>& w, bool my_eq) {
     const int t = threadIdx.x;
-    const int nb = target_buckets(key_bytes, sd.count);
+    const uint64_t my_cap = t < NB ? w.cap[t] : 0ull;
+    const uint64_t off = block_exclusive_scan_first<NB, uint64_t>(my_cap, w.wtot64, (uint64_t*)nullptr);
+    if (t < NB) {
+        out->region_off[t] = off;
+        out->region_cap[t] = my_cap;
+        // Eytzinger tree over uniq[0..254]: node i at depth d has in-order index
+        // (2*(i - 2^d) + 1) * 2^(7-d) - 1.
+        if (t >= 1) {
+            const int d = 31 - __clz(t);
+            const int io = (2 * (t - (1 << d)) + 1) * (1 << (7 - d)) - 1;
+            out->tree[t] = w.uniq[io];
+        } else {
+            out->tree[0] = KeyMax<K>::value;
+        }
+        out->uniq[t] = w.uniq[t];
+        const unsigned bal_eq = __ballot_sync(0xFFFFFFFFu, my_eq);
+        if ((t & 31) == 0) out->eq_mask[t >> 5] = bal_eq;
+        if (t < NB / 32) out->bucket_eq[t] = w.beq[t];
+    }
+}
+
+// Splitters and bucket regions of a segment of `count` keys from its m sorted
+// samples smp(0..m).  Every thread of the block calls it (a multiple of 32
+// threads, at least NB).
+template <typename K, typename Smp>
+__device__ void make_splitters(Smp smp, uint32_t m, uint64_t count, int nb, SplitSet<K>* out, SplitScratch<K>& w) {
+    const int t = threadIdx.x;
     const int ncand = nb - 1;
-    const uint32_t m = sample_size(nb);
 
     // candidate splitters at the sample quantiles
     K c = KeyMax<K>::value;
-    if (t < ncand) c = smp[(uint32_t)(((uint64_t)(t + 1) * m) / nb) - 1];
-    cand[t] = c;
+    if (t < ncand) c = smp((uint32_t)(((uint64_t)(t + 1) * m) / nb) - 1);
+    if (t < NB) w.cand[t] = c;
     __syncthreads();
     const bool valid = t < ncand;
-    const bool first = valid && (t == 0 || cand[t] != cand[t - 1]);
-    const bool dup = valid && ((t > 0 && cand[t] == cand[t - 1]) || (t + 1 < ncand && cand[t] == cand[t + 1]));
-    uint32_t j = block_exclusive_scan_first<NB, uint32_t>(first ? 1u : 0u, wtot, &total_u);
+    const bool first = valid && (t == 0 || w.cand[t] != w.cand[t - 1]);
+    const bool dup = valid && ((t > 0 && w.cand[t] == w.cand[t - 1]) || (t + 1 < ncand && w.cand[t] == w.cand[t + 1]));
+    const uint32_t j = block_exclusive_scan_first<NB, uint32_t>(first ? 1u : 0u, w.wtot, &w.total_u);
     if (first) {
-        uniq[j] = c;
-        eqf[j] = dup ? 1u : 0u;
+        w.uniq[j] = c;
+        w.eqf[j] = dup ? 1u : 0u;
     }
     __syncthreads();
-    const uint32_t K_u = total_u;
-    if (t >= (int)K_u) {
-        uniq[t] = KeyMax<K>::value;
-        eqf[t] = 0;
+    const uint32_t K_u = w.total_u;
+    if (t >= (int)K_u && t < NB) {
+        w.uniq[t] = KeyMax<K>::value;
+        w.eqf[t] = 0;
     }
     __syncthreads();
     // splitter lookup table over [sample min, sample max]
-    {
-        __shared__ uint32_t sk[NB];
-        const SlotMap<K> f = make_slot_map<K>(smp[0], smp[m - 1], (uint32_t)SPLIT_SLOTS);
-        sk[t] = t < (int)K_u ? f(uniq[t]) : 0xFFFFFFFFu;
-        if (t == 0) {
-            out->slot_map = f;
-            out->slot_hi = smp[m - 1];
-        }
-        __syncthreads();
-        auto below = [&](uint32_t s) {  // splitters with slot < s
-            uint32_t lo = 0, hi = K_u;
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (sk[mid] < s) lo = mid + 1; else hi = mid;
-            }
-            return lo;
-        };
-        for (uint32_t s = t; s < (uint32_t)SPLIT_SLOTS + 8; s += NB) {
-            const uint32_t lo = below(s);
-            const uint32_t cnt = s < (uint32_t)SPLIT_SLOTS ? below(s + 1) - lo : 0u;
-            out->slot_tab[s] = (uint16_t)(lo | (cnt << 8));
-        }
+    const SlotMap<K> f = make_slot_map_fast<K>(smp(0), smp(m - 1) - smp(0), (uint32_t)SPLIT_SLOTS);
+    if (t < NB) w.sk[t] = t < (int)K_u ? f(w.uniq[t]) : 0xFFFFFFFFu;
+    if (t == 0) {
+        out->slot_map = f;
+        out->slot_hi = smp(m - 1);
+    }
+    __syncthreads();
+    for (uint32_t s = t; s < (uint32_t)SPLIT_SLOTS + 8; s += blockDim.x) {
+        // splitters with slot < s, and those of slot s
+        const uint32_t lo = first_index(K_u, [&](uint32_t i) { return w.sk[i] >= s; });
+        uint32_t cnt = 0;
+        while (s < (uint32_t)SPLIT_SLOTS && lo + cnt < K_u && w.sk[lo + cnt] == s) ++cnt;
+        out->slot_tab[s] = (uint16_t)(lo | (cnt << 8));
     }
     // bucket ids: range_j, then eq_j if splitter j has one; the last range bucket is K_u
-    const uint32_t my_eq = (t < (int)K_u) ? eqf[t] : 0u;
-    const uint32_t eq_before = block_exclusive_scan_first<NB, uint32_t>(my_eq, wtot, &total_eq);
+    const uint32_t my_eq = (t < (int)K_u) ? w.eqf[t] : 0u;
+    const uint32_t eq_before = block_exclusive_scan_first<NB, uint32_t>(my_eq, w.wtot, &w.total_eq);
     const uint32_t range_id = (uint32_t)t + eq_before;  // valid for t <= K_u
-    if (t <= (int)K_u) out->range_b[t] = (uint8_t)range_id;
-    else out->range_b[t] = 0;
-    out->eq_b[t] = (uint8_t)(my_eq ? range_id + 1 : 0);
-    const uint32_t nbk = K_u + 1 + total_eq;
+    const uint32_t nbk = K_u + 1 + w.total_eq;
 
     // sample counts per bucket -> capacities
     // range bucket j (t <= K_u): keys in (uniq[j-1], uniq[j]] or (uniq[j-1], uniq[j]) if eq_j
-    uint64_t cap_range = 0, cap_eq = 0;
-    const double scale = (double)sd.count / (double)m;
-    auto cap_of = [&](uint32_t cnt) -> uint64_t {
-        double v = ((double)cnt + 6.0 * sqrt((double)cnt + 1.0) + 16.0) * scale;
-        uint64_t cap = (uint64_t)ceil(v);
-        if (cap > sd.count) cap = sd.count;
-        return (cap + 15) & ~15ull;
-    };
-    if (t <= (int)K_u) {
-        const uint32_t lo = (t == 0) ? 0u : upper_bound_dev<K>(smp, m, uniq[t - 1]);
-        uint32_t hi;
-        if (t == (int)K_u) hi = m;
-        else hi = my_eq ? lower_bound_dev<K>(smp, m, uniq[t]) : upper_bound_dev<K>(smp, m, uniq[t]);
-        cap_range = cap_of(hi > lo ? hi - lo : 0u);
+    const double scale = (double)count / (double)m;
+    if (t < NB) {
+        w.cap[t] = 0;
+        if (t < NB / 32) w.beq[t] = 0;
+        out->range_b[t] = t <= (int)K_u ? (uint8_t)range_id : (uint8_t)0;
+        out->eq_b[t] = (uint8_t)(my_eq ? range_id + 1 : 0);
+    }
+    __syncthreads();
+    if (t <= (int)K_u && t < NB) {
+        auto below = [&](K v) { return first_index(m, [&](uint32_t i) { return !(smp(i) < v); }); };
+        auto upto = [&](K v) { return first_index(m, [&](uint32_t i) { return v < smp(i); }); };
+        const uint32_t lo = t == 0 ? 0u : upto(w.uniq[t - 1]);
+        const uint32_t end = t == (int)K_u ? m : upto(w.uniq[t]);
+        const uint32_t hi = my_eq ? below(w.uniq[t]) : end;
+        w.cap[range_id] = bucket_cap(hi > lo ? hi - lo : 0u, scale, count);
         if (my_eq) {
-            const uint32_t e0 = lower_bound_dev<K>(smp, m, uniq[t]);
-            const uint32_t e1 = upper_bound_dev<K>(smp, m, uniq[t]);
-            cap_eq = cap_of(e1 - e0);
+            w.cap[range_id + 1] = bucket_cap(end - hi, scale, count);
+            atomicOr(&w.beq[(range_id + 1) >> 5], 1u << ((range_id + 1) & 31));
         }
     }
-    // scatter capacities into bucket order
-    if (t < NB) cap_s[t] = 0;
     __syncthreads();
-    if (t <= (int)K_u) {
-        cap_s[range_id] = cap_range;
-        if (my_eq) cap_s[range_id + 1] = cap_eq;
-    }
-    __syncthreads();
-    const uint64_t my_cap = cap_s[t];
-    const uint64_t off = block_exclusive_scan_first<NB, uint64_t>(my_cap, wtot64, &cap_total);
-    out->region_off[t] = off;
-    out->region_cap[t] = my_cap;
-    // Eytzinger tree over uniq[0..254]: node i at depth d has in-order index
-    // (2*(i - 2^d) + 1) * 2^(7-d) - 1.
-    if (t >= 1 && t < NB) {
-        const int d = 31 - __clz(t);
-        const int io = (2 * (t - (1 << d)) + 1) * (1 << (7 - d)) - 1;
-        out->tree[t] = uniq[io];
-    } else {
-        out->tree[0] = KeyMax<K>::value;
-    }
-    out->uniq[t] = uniq[t];
-    // masks
-    const unsigned bal_eq = __ballot_sync(0xFFFFFFFFu, my_eq != 0);
-    if ((t & 31) == 0) out->eq_mask[t >> 5] = bal_eq;
-    __shared__ uint32_t beq[NB / 32];
-    if (t < NB / 32) beq[t] = 0;
-    __syncthreads();
-    if (my_eq) atomicOr(&beq[(range_id + 1) >> 5], 1u << ((range_id + 1) & 31));
-    __syncthreads();
-    if (t < NB / 32) out->bucket_eq[t] = beq[t];
+    write_layout<K>(out, w, my_eq != 0);
     if (t == 0) {
         out->nbuckets = nbk;
-        out->has_eq = total_eq ? 1u : 0u;
+        out->has_eq = w.total_eq ? 1u : 0u;
         out->nuniq = K_u;
+        out->direct = 0;
     }
+}
+
+// The splitters of a sorted sample in global memory (one segment per block).
+template <typename K>
+__global__ void __launch_bounds__(NB) splitter_kernel(const K* __restrict__ samples, const SegDesc* __restrict__ segs,
+                                                      uint32_t nsegs, SplitSet<K>* __restrict__ splits,
+                                                      int key_bytes) {
+    __shared__ SplitScratch<K> w;
+    const uint32_t s = blockIdx.x;
+    if (s >= nsegs) return;
+    const K* smp = samples + (size_t)s * SAMPLE_N;
+    const uint64_t count = segs[s].count;
+    const int nb = target_buckets(key_bytes, count);
+    make_splitters<K>([&](uint32_t i) { return smp[i]; }, sample_size(nb), count, nb, splits + s, w);
+}
+
+// Split a segment at slot boundaries, from the histogram of its samples over
+// the slots: no sort, no splitter search, and the partition pass finds a key's
+// bucket with one table byte.  A slot goes to the bucket that the middle of
+// its samples falls in (in rank), so bucket ids rise with the slots.  Returns
+// false, with nothing written, when the sample is not spread finely enough
+// over the slots: a slot that holds half a bucket's share (repeated values,
+// clusters) would leave uneven buckets and needs splitters between keys.
+// `smem` holds DIRECT_SLOTS counters, then the scratch.  Every thread calls it.
+template <typename K, int THREADS, int IPT>
+__device__ bool make_direct(const K (&key)[IPT], uint32_t m, uint64_t count, int nb, SplitSet<K>* out,
+                            unsigned char* smem, SlotRed<K>& red) {
+    constexpr int PER = DIRECT_SLOTS / THREADS;  // slots per thread
+    static_assert(PER == 16, "a thread writes its slots' table bytes as one 16-byte word");
+    struct Scratch {
+        SplitScratch<K> w;
+        uint32_t first_slot[NB + 1], rank0[NB + 1];  // per bucket: its first slot, the samples before it
+        uint8_t last[THREADS];                       // per thread: the bucket of its last slot
+    };
+    unsigned char* hist = smem;
+    Scratch& d = *reinterpret_cast<Scratch*>(smem + DIRECT_SLOTS * sizeof(uint32_t));
+    const unsigned t = threadIdx.x, lane = lane_id(), warp = t >> 5;
+    auto quad = [&](int j) {
+        return reinterpret_cast<uint4*>(hist + ctr_swizzle<PER>(t * PER * 4 + (uint32_t)j * 16));
+    };
+#pragma unroll
+    for (int j = 0; j < PER / 4; ++j) *quad(j) = make_uint4(0u, 0u, 0u, 0u);
+    K lo, range;
+    block_bounds<K, THREADS, IPT>(key, m, red, lo, range);
+    const SlotMap<K> f = make_slot_map_fast<K>(lo, range, (uint32_t)DIRECT_SLOTS);
+    if (f.direct) return false;  // fewer values than slots
+    DirectMap<K> dm;
+    dm.lo = lo;
+    dm.sh = f.sh;
+    dm.mul = f.mul;
+    dm.dmax = (uint32_t)(range >> f.sh);
+    dm.hmax = sizeof(K) == 8 ? (uint32_t)((uint64_t)range >> 32) : 0u;
+    const uint32_t most = m / (uint32_t)nb / 2;  // samples allowed in a slot
+    bool heavy = false;
+#pragma unroll
+    for (int r = 0; r < IPT; ++r) {
+        if ((uint32_t)r * THREADS + t < m) {
+            bool unused = false;
+            const uint32_t a = ctr_swizzle<PER>(dm.fast(key[r], unused) * 4u);
+            heavy |= atomicAdd(reinterpret_cast<uint32_t*>(hist + a), 1u) >= most;
+        }
+    }
+    if (__syncthreads_or(heavy)) return false;
+
+    // samples before each slot, and from them its bucket
+    uint32_t sum = 0;
+#pragma unroll
+    for (int j = 0; j < PER / 4; ++j) {
+        const uint4 q = *quad(j);
+        sum += q.x + q.y + q.z + q.w;
+    }
+    uint32_t inc = sum;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, inc, k);
+        if (lane >= (unsigned)k) inc += o;
+    }
+    if (lane == 31) red.wtot[warp] = inc;
+    if (t <= NB) {  // buckets that no slot starts are empty
+        d.first_slot[t] = DIRECT_SLOTS;
+        d.rank0[t] = m;
+    }
+    if (t < NB / 32) d.w.beq[t] = 0;
+    __syncthreads();
+    uint32_t run = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? red.wtot[lane] : 0u) + inc - sum;
+    const float per_rank = (float)nb / (float)(2 * m);
+    // (counts below 2^15 and their products are exact enough in float that a
+    // larger rank never gives a smaller bucket: the product is monotone)
+    auto bucket = [&](uint32_t before, uint32_t c) {
+        return min((uint32_t)((float)(2 * before + c) * per_rank), (uint32_t)(nb - 1));
+    };
+    uint32_t rank[PER], bk[PER];
+#pragma unroll
+    for (int j = 0; j < PER / 4; ++j) {
+        const uint4 q = *quad(j);
+        const uint32_t c[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            rank[4 * j + k] = run;
+            bk[4 * j + k] = bucket(run, c[k]);
+            run += c[k];
+        }
+    }
+    uint32_t pack[PER / 4];
+#pragma unroll
+    for (int j = 0; j < PER / 4; ++j)
+        pack[j] = bk[4 * j] | (bk[4 * j + 1] << 8) | (bk[4 * j + 2] << 16) | (bk[4 * j + 3] << 24);
+    reinterpret_cast<uint4*>(out->dir_tab)[t] = make_uint4(pack[0], pack[1], pack[2], pack[3]);
+    d.last[t] = (uint8_t)bk[PER - 1];
+    __syncthreads();
+    uint32_t prev = t ? d.last[t - 1] : 0u;
+    if (t == 0) {
+        d.first_slot[0] = 0;
+        d.rank0[0] = 0;
+    }
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        for (; prev < bk[k]; ++prev) {
+            d.first_slot[prev + 1] = t * PER + k;
+            d.rank0[prev + 1] = rank[k];
+        }
+    }
+    __syncthreads();
+    if (t < NB) {
+        const bool live = t < (unsigned)nb;
+        d.w.cap[t] = live ? bucket_cap(d.rank0[t + 1] - d.rank0[t], (double)count / (double)m, count) : 0ull;
+        // splitter t: the last key before bucket t + 1 (slot 0 is always in
+        // bucket 0: it holds less than half a bucket's samples)
+        const uint32_t s = t + 1 < (unsigned)nb ? d.first_slot[t + 1] : (uint32_t)DIRECT_SLOTS;
+        d.w.uniq[t] = s <= dm.slot(lo + range) ? dm.first_key(s) - 1 : KeyMax<K>::value;
+        out->range_b[t] = live ? (uint8_t)t : (uint8_t)0;
+        out->eq_b[t] = 0;
+    }
+    __syncthreads();
+    write_layout<K>(out, d.w, false);
+    if (t == 0) {
+        out->nbuckets = (uint32_t)nb;
+        out->has_eq = 0;
+        out->nuniq = (uint32_t)nb - 1;
+        out->direct = 1;
+        out->dir_map = dm;
+    }
+    return true;
+}
+
+// Keys sampled from every segment, `parts` blocks per segment: random reads
+// are bound by how many one SM can have outstanding, so they are spread over
+// the chip (16384 reads by one block take 13 us to 33 us, by 64 blocks 2.2 us).
+template <typename Codec>
+__global__ void __launch_bounds__(256) sample_kernel(Codec in, const SegDesc* __restrict__ segs, uint32_t parts,
+                                                     typename Codec::Key* __restrict__ samples, uint64_t seed,
+                                                     int key_bytes) {
+    const uint32_t s = blockIdx.x / parts, part = blockIdx.x % parts;
+    const uint64_t in_off = segs[s].in_off, count = segs[s].count;
+    const uint32_t m = sample_size(target_buckets(key_bytes, count));
+#pragma unroll 4
+    for (uint32_t i = part * 256 + threadIdx.x; i < m; i += parts * 256)
+        samples[(size_t)s * SAMPLE_N + i] =
+            in.load(in_off + __umul64hi(mix64(seed ^ ((uint64_t)s << 32) ^ (uint64_t)i), count));
+}
+
+// Splitters and regions of every segment from its samples: one block of 1024
+// threads per segment.  The work is a chain of latencies on one SM, so the
+// sort of the sample is left out where its histogram will do (make_direct),
+// and searches run in shared memory.  Sampling to splitters for one segment:
+// int32 52 -> 11 us, 64-bit keys 58 -> 15 us; for the 256 segments of the
+// second level of 2^28 doubles 165 -> 125 us (three kernels before, the
+// sample sorted, written out and searched in L2).
+constexpr int SAMPLE_THREADS = 1024;
+constexpr int SAMPLE_IPT = SAMPLE_N / SAMPLE_THREADS;
+template <typename K>
+constexpr size_t split_smem() { return SlotSmem<K, SAMPLE_THREADS, SAMPLE_IPT>::bytes; }
+
+template <typename K>
+__global__ void __launch_bounds__(SAMPLE_THREADS)
+    split_kernel(K* __restrict__ samples, const SegDesc* __restrict__ segs, SplitSet<K>* __restrict__ splits,
+                 int key_bytes, int keep_sorted) {
+    using SM = SlotSmem<K, SAMPLE_THREADS, SAMPLE_IPT>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ SlotRed<K> red;
+    const uint32_t s = blockIdx.x;
+    const uint64_t count = segs[s].count;
+    const int nb = target_buckets(key_bytes, count);
+    const uint32_t m = sample_size(nb);
+    K* g = samples + (size_t)s * SAMPLE_N;
+    K key[SAMPLE_IPT];
+#pragma unroll
+    for (int r = 0; r < SAMPLE_IPT; ++r) {
+        const uint32_t i = (uint32_t)r * SAMPLE_THREADS + threadIdx.x;
+        if (i < m) key[r] = g[i];
+    }
+    if (make_direct<K, SAMPLE_THREADS, SAMPLE_IPT>(key, m, count, nb, splits + s, smem_raw, red)) return;
+    __syncthreads();
+    const K any = key[0];  // (m >= SAMPLE_THREADS)
+    // sorted in registers and shared memory, where the splitters are searched;
+    // back to global memory only for the learned fit
+    const SlotPath how = block_slot_sort<K, SAMPLE_THREADS, SAMPLE_IPT, true>(
+        key, m, [&](uint32_t i, K x) { if (keep_sorted) g[i] = x; }, [] {}, [] {}, smem_raw, red);
+    __syncthreads();
+    const K* sorted = reinterpret_cast<const K*>(smem_raw);
+    static_assert(sizeof(SplitScratch<K>) <= SM::ctr_bytes, "the counters' space is reused");
+    SplitScratch<K>& w = *reinterpret_cast<SplitScratch<K>*>(smem_raw + SM::keys_bytes);
+    make_splitters<K>(
+        [&](uint32_t i) { return how == SLOT_EQUAL ? any : sorted[how == SLOT_EVEN ? i : pidx(i)]; }, m, count, nb,
+        splits + s, w);
 }
 
 // Bucket of key x under a split set held in shared memory.
@@ -415,6 +611,13 @@ namespace s512 {
 // ===========================================================================
 // 4. The partition pass (persistent; tiles claimed in runs)
 //
+// What bounds it: issue slots and the shared-memory pipe (wavefronts), not HBM,
+// so the classification is kept short: a segment split at slot boundaries
+// (ROUTE_DIRECT) needs a subtraction, a shift, a multiply and one table byte
+// per key.  One 256-way pass over 2^28 doubles: 1.58 ms when every key was
+// clamped, looked up and compared with the splitters of its slot, 1.25 ms
+// (level 0) and 1.64 -> 1.38 ms (level 1) direct; the floor is 0.66 ms.
+//
 // Every tile of keys is classified, ranked within the tile by shared-memory
 // atomics, staged in bucket order in shared memory and written out with
 // coalesced stores.  Where a tile's keys of bucket b go inside the bucket's
@@ -476,6 +679,16 @@ struct PlainTables {
     alignas(16) uint16_t tab[SPLIT_SLOTS + 8];
 };
 
+// The routing table of a segment split at slot boundaries.
+template <typename K>
+struct DirectTables {
+    DirectMap<K> map;
+    alignas(16) uint8_t tab[DIRECT_SLOTS];
+};
+
+// What finds the bucket of a segment's keys.
+enum : uint32_t { ROUTE_SPLIT = 0, ROUTE_LEARNED = 1, ROUTE_DIRECT = 2 };
+
 // Bytes of a LearnedSet that inference reads (its leading fields).
 template <typename K>
 constexpr size_t learned_model_bytes() { return offsetof(LearnedSet<K>, region_off); }
@@ -487,18 +700,19 @@ struct PartSmem {
     uint8_t bkt[TILE];
     uint64_t region_off[NB];
     uint64_t region_cap[NB];
-    uint64_t gdelta[NB];
+    uint64_t gptr[NB];            // bucket b's keys of the tile: position p goes to (K*)gptr[b] + p
     uint32_t hist[NB];
     uint32_t loc[NB];
     uint32_t seg_tile_start[SEG_SMEM];
     uint64_t mbar[2];
-    uint32_t tile_cur, has_eq, use_learned, abort;
+    uint32_t tile_cur, has_eq, route, abort;
     SegDesc sd;                   // segment of the tile being processed
     SegDesc iss_sd;               // thread 0: segment of the last tile it fetched
     uint32_t iss_seg;
-    // a segment routes by its split set or by its learned model, never both
+    // a segment routes by one of these
     union {
         PlainTables<K> P;
+        DirectTables<K> D;
         alignas(16) unsigned char model[learned_model_bytes<K>()];
     } T;
 };
@@ -511,7 +725,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) partition_kernel(Part
     constexpr int TILE = THREADS * IPT;
     constexpr int ESZ = InCodec::ESZ;
     constexpr int NARR = InCodec::NARR;
-    static_assert(TILE < (1 << 24), "rank and bucket share a 32-bit word");
+    static_assert(TILE < (1 << 21), "rank and bucket share a 32-bit word");
     static_assert(TILE <= (int)JUNK_KEYS, "an overflowed bucket's keys of a tile fit the overflow area");
     const int tid = threadIdx.x;
     const uint32_t ntiles = a.ntiles_dev ? *a.ntiles_dev : a.ntiles;
@@ -597,8 +811,20 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) partition_kernel(Part
             // tiles (the previous tile's write-out reads none of them)
             if (tid < (int)(sizeof(SegDesc) / 4))
                 reinterpret_cast<uint32_t*>(&sm.sd)[tid] = reinterpret_cast<const uint32_t*>(&a.segs[seg])[tid];
-            const bool use_learned = a.learned && a.learned[seg].ok;
-            if (use_learned) {
+            const uint32_t route = a.learned && a.learned[seg].ok ? ROUTE_LEARNED
+                                   : a.splits[seg].direct         ? ROUTE_DIRECT
+                                                                  : ROUTE_SPLIT;
+            if (route == ROUTE_DIRECT) {
+                const SplitSet<K>& ss = a.splits[seg];
+                for (int i = tid; i < NB; i += THREADS) {
+                    sm.region_off[i] = ss.region_off[i];
+                    sm.region_cap[i] = ss.region_cap[i];
+                }
+                const uint4* src = reinterpret_cast<const uint4*>(ss.dir_tab);
+                uint4* dst = reinterpret_cast<uint4*>(sm.T.D.tab);
+                for (int i = tid; i < DIRECT_SLOTS / 16; i += THREADS) dst[i] = src[i];
+                if (tid == 0) sm.T.D.map = ss.dir_map;
+            } else if (route == ROUTE_LEARNED) {
                 const LearnedSet<K>& ls = a.learned[seg];
                 const uint32_t* src = reinterpret_cast<const uint32_t*>(&ls);
                 uint32_t* dst = reinterpret_cast<uint32_t*>(sm.T.model);
@@ -628,7 +854,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) partition_kernel(Part
                     sm.T.P.fhi = ss.slot_hi;
                 }
             }
-            if (tid == 0) sm.use_learned = use_learned ? 1u : 0u;
+            if (tid == 0) sm.route = route;
             cached_seg = seg;
         }
         bool data_ok = true;
@@ -654,9 +880,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) partition_kernel(Part
         const uint64_t rem = sm.sd.count - (uint64_t)ti * TILE;
         const uint32_t cnt = rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
         const uint32_t tma_elems = a.tma ? ((cnt * ESZ) & ~15u) / ESZ : 0u;
-        const bool has_eq = sm.has_eq != 0;
-        const bool learned = sm.use_learned != 0;
-        const SlotRegs<K> fm(sm.T.P.fmap, sm.T.P.fhi);  // (meaningless for a learned segment: unused)
+        const uint32_t route = sm.route;
 
         // a whole tile from the bulk copy (no per-key range checks)
         const bool FULL = cnt == (uint32_t)TILE && tma_elems == (uint32_t)TILE;
@@ -665,7 +889,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) partition_kernel(Part
             // tile; tail elements past the copied bytes from global memory),
             // their buckets and their ranks within the tile
             K key[IPT];
-            uint32_t br[IPT];  // bucket | rank << 8
+            uint32_t br[IPT];  // 4 * bucket | rank << 11
 #pragma unroll
             for (int r = 0; r < IPT; ++r) {
                 const uint32_t idx = (uint32_t)(r * THREADS + tid);
@@ -673,54 +897,72 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) partition_kernel(Part
                 else if (idx < cnt) key[r] = idx < tma_elems ? in.decode(sm.buf[b], idx, TILE) : in.load(base + idx);
             }
             // all IPT bucket lookups first: they are independent chains of
-            // shared loads, so the scheduler can overlap them
-            uint32_t bks[IPT];
-            if (learned) {
+            // shared loads, so the scheduler can overlap them.  (Lanes past
+            // the end look up stale register contents, in bounds, and then
+            // carry the out-of-range bucket NB.)
+            if (route == ROUTE_DIRECT) {
+                const DirectMap<K> dm = sm.T.D.map;
+                bool out = false;
+#pragma unroll
+                for (int r = 0; r < IPT; ++r) br[r] = dm.fast(key[r], out);
+                if (out) {  // a key outside the sample's range (2 in 16384 or so)
+#pragma unroll
+                    for (int r = 0; r < IPT; ++r) br[r] = dm.slot(key[r]);
+                }
+#pragma unroll
+                for (int r = 0; r < IPT; ++r) br[r] = (uint32_t)sm.T.D.tab[br[r]] << 2;
+            } else if (route == ROUTE_LEARNED) {
 #pragma unroll
                 for (int r = 0; r < IPT; ++r) {
                     const uint32_t idx = (uint32_t)(r * THREADS + tid);
                     // (only the model prefix of the LearnedSet is in shared memory)
-                    bks[r] = (FULL || idx < cnt)
-                                 ? learned_bucket<K>(*reinterpret_cast<const LearnedSet<K>*>(sm.T.model), key[r])
-                                 : (uint32_t)NB;  // lanes past the end carry the out-of-range bucket NB
+                    if (FULL || idx < cnt)
+                        br[r] = learned_bucket<K>(*reinterpret_cast<const LearnedSet<K>*>(sm.T.model), key[r]) << 2;
                 }
             } else {
+                const bool has_eq = sm.has_eq != 0;
+                const SlotRegs<K> fm(sm.T.P.fmap, sm.T.P.fhi);
 #pragma unroll
-                for (int r = 0; r < IPT; ++r) bks[r] = sm.T.P.tab[fm(key[r])];  // slot entries first
+                for (int r = 0; r < IPT; ++r) br[r] = sm.T.P.tab[fm(key[r])];  // slot entries first
 #pragma unroll
                 for (int r = 0; r < IPT; ++r) {
                     const uint32_t idx = (uint32_t)(r * THREADS + tid);
-                    bks[r] = (FULL || idx < cnt) ? bucket_from_slot<K>(bks[r], key[r], has_eq, sm.T.P.uniq,
-                                                                       sm.T.P.range_b, sm.T.P.eq_b, sm.T.P.eq_mask)
-                                                 : (uint32_t)NB;
+                    if (FULL || idx < cnt)
+                        br[r] = bucket_from_slot<K>(br[r], key[r], has_eq, sm.T.P.uniq, sm.T.P.range_b, sm.T.P.eq_b,
+                                                    sm.T.P.eq_mask) << 2;
                 }
             }
+            if (!FULL) {
+#pragma unroll
+                for (int r = 0; r < IPT; ++r)
+                    if ((uint32_t)(r * THREADS + tid) >= cnt) br[r] = 4u * NB;
+            }
+            auto hist = [&](uint32_t b4) { return reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(sm.hist) + b4); };
             // A warp whose 32 keys share a bucket (sorted or constant runs)
             // ranks them with one atomic instead of 32 on one address.  Whether
             // to look for that is decided once per tile from the warp's first
             // 32 keys: on unsorted input the check would cost a shuffle and a
             // vote per key and never pay.
-            const bool try_uni = __all_sync(0xFFFFFFFFu, bks[0] == __shfl_sync(0xFFFFFFFFu, bks[0], 0));
+            if (__all_sync(0xFFFFFFFFu, br[0] == __shfl_sync(0xFFFFFFFFu, br[0], 0))) {
 #pragma unroll
-            for (int r = 0; r < IPT; ++r) {
-                const uint32_t bk = bks[r];
-                uint32_t b0 = bk;
-                bool uni = false;
-                if (try_uni) {
-                    b0 = __shfl_sync(0xFFFFFFFFu, bk, 0);
-                    uni = __all_sync(0xFFFFFFFFu, bk == b0);
-                }
-                uint32_t rank = 0;
-                if (uni) {
-                    if (FULL || b0 < (uint32_t)NB) {
-                        uint32_t basev = 0;
-                        if (lane_id() == 0) basev = atomicAdd(&sm.hist[b0], 32u);
-                        rank = __shfl_sync(0xFFFFFFFFu, basev, 0) + lane_id();
+                for (int r = 0; r < IPT; ++r) {
+                    const uint32_t b0 = __shfl_sync(0xFFFFFFFFu, br[r], 0);
+                    uint32_t rank = 0;
+                    if (__all_sync(0xFFFFFFFFu, br[r] == b0)) {
+                        if (b0 < 4u * NB) {
+                            uint32_t basev = 0;
+                            if (lane_id() == 0) basev = atomicAdd(hist(b0), 32u);
+                            rank = __shfl_sync(0xFFFFFFFFu, basev, 0) + lane_id();
+                        }
+                    } else if (br[r] < 4u * NB) {
+                        rank = atomicAdd(hist(br[r]), 1u);
                     }
-                } else if (FULL || bk < (uint32_t)NB) {
-                    rank = atomicAdd(&sm.hist[bk], 1u);
+                    br[r] |= rank << 11;
                 }
-                br[r] = bk | (rank << 8);
+            } else {
+#pragma unroll
+                for (int r = 0; r < IPT; ++r)
+                    if (FULL || br[r] < 4u * NB) br[r] |= atomicAdd(hist(br[r]), 1u) << 11;
             }
             __syncthreads();  // (1) the tile's histogram is complete; the previous tile is written
 
@@ -765,18 +1007,19 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) partition_kernel(Part
             for (int r = 0; r < IPT; ++r) {
                 const uint32_t idx = (uint32_t)(r * THREADS + tid);
                 if (FULL || idx < cnt) {
-                    const uint32_t bk = br[r] & 0xFFu;
-                    const uint32_t p = sm.loc[bk] + (br[r] >> 8);
+                    const uint32_t p =
+                        *reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(sm.loc) + (br[r] & 0x7FCu)) +
+                        (br[r] >> 11);
                     stage[p] = key[r];
-                    sm.bkt[p] = (uint8_t)bk;
+                    sm.bkt[p] = (uint8_t)(br[r] >> 2);
                 }
             }
             if (tid < NB) {
                 const unsigned long long end = off + h;
                 const bool ovf = !data_ok || end > sm.region_cap[tid];
                 if (ovf && h) raise_error(&a.ctl->err, data_ok ? DEV_ERR_OVERFLOW : DEV_ERR_TIMEOUT);
-                sm.gdelta[tid] =
-                    (ovf ? a.junk : sm.sd.out_base + sm.region_off[tid] + off) - (uint64_t)sm.loc[tid];
+                sm.gptr[tid] = reinterpret_cast<uint64_t>(
+                    a.out + (ovf ? a.junk : sm.sd.out_base + sm.region_off[tid] + off) - sm.loc[tid]);
                 sm.hist[tid] = 0;  // (next used after barrier (3))
             }
             if (tid == 0 && !data_ok) sm.abort = 1;
@@ -787,10 +1030,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) partition_kernel(Part
 #pragma unroll
             for (int r = 0; r < IPT; ++r) {
                 const uint32_t i = (uint32_t)(r * THREADS + tid);
-                if (FULL || i < cnt) {
-                    const uint64_t g = sm.gdelta[sm.bkt[i]];
-                    a.out[g + i] = stage[i];
-                }
+                if (FULL || i < cnt) reinterpret_cast<K*>(sm.gptr[sm.bkt[i]])[i] = stage[i];
             }
         }
         b ^= 1;
