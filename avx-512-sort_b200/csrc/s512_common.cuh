@@ -48,10 +48,11 @@ __device__ __forceinline__ uint32_t enc_i32(int x) { return (uint32_t)x ^ 0x8000
 __device__ __forceinline__ int dec_i32(uint32_t k) { return (int)(k ^ 0x80000000u); }
 
 __device__ __forceinline__ uint64_t enc_f64_bits(uint64_t u) {
-    return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
+    // (the sign smeared over the word: three operations on 32-bit halves)
+    return u ^ ((uint64_t)((int64_t)u >> 63) | 0x8000000000000000ull);
 }
 __device__ __forceinline__ uint64_t dec_f64_bits(uint64_t k) {
-    return (k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFull) : ~k;
+    return k ^ (~(uint64_t)((int64_t)k >> 63) | 0x8000000000000000ull);
 }
 
 // key in the high half, value in the low half, both in signed order, so that
@@ -66,74 +67,60 @@ __device__ __forceinline__ uint64_t enc_kv(int key, int val) {
 //   store(i, k)  -> write encoded key k as element i of the destination
 // `Raw` is the identity codec used on the library's own scratch buffers.
 
-// Besides load/store, every input codec describes its raw arrays (NARR
-// arrays of ESZ-byte elements, arr(k)) and decodes element i of a tile that a
-// bulk copy placed in shared memory (array k of the tile at buf + k*tile*ESZ).
+// Input codecs also split load(i) into raw(i), the element's bits as they are
+// stored, and enc(bits): a kernel that loads ahead keeps the bits, so that
+// nothing waits for them before they are needed.
 template <typename K>
 struct Raw {
     using Key = K;
-    static constexpr int NARR = 1;
-    static constexpr int ESZ = sizeof(K);
     const K* __restrict__ in;
     K* __restrict__ out;
+    __device__ __forceinline__ K raw(size_t i) const { return __ldg(in + i); }
+    static __device__ __forceinline__ K enc(K w) { return w; }
     __device__ __forceinline__ K load(size_t i) const { return __ldg(in + i); }
     __device__ __forceinline__ void store(size_t i, K k) const { out[i] = k; }
-    __host__ __device__ const void* arr(int) const { return in; }
     // the same codec reading other arrays (e.g. the caller's page-locked host memory)
     Raw rebased(const void* const* a) const { return Raw{static_cast<const K*>(a[0]), out}; }
-    __device__ __forceinline__ K decode(const unsigned char* buf, uint32_t i, uint32_t) const {
-        return reinterpret_cast<const K*>(buf)[i];
-    }
 };
 
 struct CodecI32 {
     using Key = uint32_t;
-    static constexpr int NARR = 1;
-    static constexpr int ESZ = 4;
     const int* __restrict__ in;
     int* __restrict__ out;
-    __device__ __forceinline__ uint32_t load(size_t i) const { return enc_i32(__ldg(in + i)); }
+    __device__ __forceinline__ uint32_t raw(size_t i) const { return (uint32_t)__ldg(in + i); }
+    static __device__ __forceinline__ uint32_t enc(uint32_t w) { return enc_i32((int)w); }
+    __device__ __forceinline__ uint32_t load(size_t i) const { return enc(raw(i)); }
     __device__ __forceinline__ void store(size_t i, uint32_t k) const { out[i] = dec_i32(k); }
-    __host__ __device__ const void* arr(int) const { return in; }
     CodecI32 rebased(const void* const* a) const { return CodecI32{static_cast<const int*>(a[0]), out}; }
-    __device__ __forceinline__ uint32_t decode(const unsigned char* buf, uint32_t i, uint32_t) const {
-        return enc_i32(reinterpret_cast<const int*>(buf)[i]);
-    }
 };
 
 struct CodecF64 {
     using Key = uint64_t;
-    static constexpr int NARR = 1;
-    static constexpr int ESZ = 8;
     const unsigned long long* __restrict__ in;
     unsigned long long* __restrict__ out;
-    __device__ __forceinline__ uint64_t load(size_t i) const { return enc_f64_bits(__ldg(in + i)); }
+    __device__ __forceinline__ uint64_t raw(size_t i) const { return __ldg(in + i); }
+    static __device__ __forceinline__ uint64_t enc(uint64_t w) { return enc_f64_bits(w); }
+    __device__ __forceinline__ uint64_t load(size_t i) const { return enc(raw(i)); }
     __device__ __forceinline__ void store(size_t i, uint64_t k) const { out[i] = dec_f64_bits(k); }
-    __host__ __device__ const void* arr(int) const { return in; }
     CodecF64 rebased(const void* const* a) const {
         return CodecF64{static_cast<const unsigned long long*>(a[0]), out};
-    }
-    __device__ __forceinline__ uint64_t decode(const unsigned char* buf, uint32_t i, uint32_t) const {
-        return enc_f64_bits(reinterpret_cast<const unsigned long long*>(buf)[i]);
     }
 };
 
 struct CodecKV {
     using Key = uint64_t;
-    static constexpr int NARR = 2;
-    static constexpr int ESZ = 4;
     const int* __restrict__ kin;
     const int* __restrict__ vin;
     int* __restrict__ kout;
     int* __restrict__ vout;
-    __host__ __device__ const void* arr(int k) const { return k ? (const void*)vin : (const void*)kin; }
     CodecKV rebased(const void* const* a) const {
         return CodecKV{static_cast<const int*>(a[0]), static_cast<const int*>(a[1]), kout, vout};
     }
-    __device__ __forceinline__ uint64_t decode(const unsigned char* buf, uint32_t i, uint32_t tile) const {
-        return enc_kv(reinterpret_cast<const int*>(buf)[i], reinterpret_cast<const int*>(buf + (size_t)tile * 4)[i]);
+    __device__ __forceinline__ uint64_t raw(size_t i) const {
+        return ((uint64_t)(uint32_t)__ldg(kin + i) << 32) | (uint32_t)__ldg(vin + i);
     }
-    __device__ __forceinline__ uint64_t load(size_t i) const { return enc_kv(__ldg(kin + i), __ldg(vin + i)); }
+    static __device__ __forceinline__ uint64_t enc(uint64_t w) { return w ^ 0x8000000080000000ull; }
+    __device__ __forceinline__ uint64_t load(size_t i) const { return enc(raw(i)); }
     __device__ __forceinline__ void store(size_t i, uint64_t k) const {
         kout[i] = dec_i32((uint32_t)(k >> 32));
         vout[i] = dec_i32((uint32_t)k);
@@ -143,18 +130,14 @@ struct CodecKV {
 // int64 keys: uint64 k = x ^ 2^63 (signed order).
 struct CodecI64 {
     using Key = uint64_t;
-    static constexpr int NARR = 1;
-    static constexpr int ESZ = 8;
     const unsigned long long* __restrict__ in;
     unsigned long long* __restrict__ out;
-    __device__ __forceinline__ uint64_t load(size_t i) const { return __ldg(in + i) ^ 0x8000000000000000ull; }
+    __device__ __forceinline__ uint64_t raw(size_t i) const { return __ldg(in + i); }
+    static __device__ __forceinline__ uint64_t enc(uint64_t w) { return w ^ 0x8000000000000000ull; }
+    __device__ __forceinline__ uint64_t load(size_t i) const { return enc(raw(i)); }
     __device__ __forceinline__ void store(size_t i, uint64_t k) const { out[i] = k ^ 0x8000000000000000ull; }
-    __host__ __device__ const void* arr(int) const { return in; }
     CodecI64 rebased(const void* const* a) const {
         return CodecI64{static_cast<const unsigned long long*>(a[0]), out};
-    }
-    __device__ __forceinline__ uint64_t decode(const unsigned char* buf, uint32_t i, uint32_t) const {
-        return reinterpret_cast<const unsigned long long*>(buf)[i] ^ 0x8000000000000000ull;
     }
 };
 
@@ -162,25 +145,20 @@ struct CodecI64 {
 // word per pair (little-endian: key in the low half), encoded like CodecKV.
 struct CodecKVPairs {
     using Key = uint64_t;
-    static constexpr int NARR = 1;
-    static constexpr int ESZ = 8;
     const unsigned long long* __restrict__ in;
     unsigned long long* __restrict__ out;
-    static __device__ __forceinline__ uint64_t enc(unsigned long long w) {
+    __device__ __forceinline__ uint64_t raw(size_t i) const { return __ldg(in + i); }
+    static __device__ __forceinline__ uint64_t enc(uint64_t w) {
         return enc_kv((int)(uint32_t)w, (int)(uint32_t)(w >> 32));
     }
-    __device__ __forceinline__ uint64_t load(size_t i) const { return enc(__ldg(in + i)); }
+    __device__ __forceinline__ uint64_t load(size_t i) const { return enc(raw(i)); }
     __device__ __forceinline__ void store(size_t i, uint64_t k) const {
         const uint32_t key = (uint32_t)dec_i32((uint32_t)(k >> 32));
         const uint32_t val = (uint32_t)dec_i32((uint32_t)k);
         out[i] = ((unsigned long long)val << 32) | key;
     }
-    __host__ __device__ const void* arr(int) const { return in; }
     CodecKVPairs rebased(const void* const* a) const {
         return CodecKVPairs{static_cast<const unsigned long long*>(a[0]), out};
-    }
-    __device__ __forceinline__ uint64_t decode(const unsigned char* buf, uint32_t i, uint32_t) const {
-        return enc(reinterpret_cast<const unsigned long long*>(buf)[i]);
     }
 };
 
@@ -243,66 +221,6 @@ __device__ __forceinline__ unsigned long long ld_status(const unsigned long long
 __device__ __forceinline__ void st_status(unsigned long long* p, unsigned long long v) {
     cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> r(*p);
     r.store(v, cuda::memory_order_relaxed);
-}
-
-// ---------------------------------------------------------------------------
-// 1-D bulk copies (TMA, no multicast) completing on a CTA mbarrier
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() {
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-// order earlier generic-proxy accesses of shared memory before later
-// async-proxy (bulk copy) writes to it
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-// dst, src 16-byte aligned; bytes a positive multiple of 16
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t phase) {
-    uint32_t ok;
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(phase)
-        : "memory");
-    return ok != 0;
-}
-// try_wait that suspends the thread in hardware until the phase completes or
-// `ns` nanoseconds pass (instead of returning at once): a waiting warp takes
-// no issue slots from the other warps of the SM
-__device__ __forceinline__ bool mbar_try_wait_suspend(uint64_t* bar, uint32_t phase, uint32_t ns) {
-    uint32_t ok;
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(phase), "r"(ns)
-        : "memory");
-    return ok != 0;
-}
-// Iterations of a suspending wait: at most about a second in all.
-constexpr uint32_t SUSPEND_NS = 1000;
-constexpr uint32_t SUSPEND_LIMIT = 1u << 20;
-
-// bounded wait for a phase of an mbarrier; false if the limit was reached
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t phase) {
-    for (uint32_t i = 0; i < SUSPEND_LIMIT; ++i)
-        if (mbar_try_wait_suspend(bar, phase, SUSPEND_NS)) return true;
-    return false;
 }
 
 // splitmix64 finaliser: counter-based hashing for sample positions

@@ -8,6 +8,8 @@
 //   p0  = c[s] + w[s] * min(zr - s, 1),   s = min(floor(zr), R - 1)   (root)
 //   l   = clamp(floor(p0 * LEAVES))                           (leaf choice)
 //   p   = clamp(a[l] + b[l] * float(key - base[l]), lo[l], hi[l])
+//   bucket = cal[min(floor(p * CELLS), CELLS - 1)]            (calibrated), or,
+//            with heavy keys among the splitters,
 //   r   = min(floor(p * nmodel), nmodel - 1)                  (model bucket)
 // with w = theta^2 >= 0 (root slopes; each trimmed so that c[s] + w[s] <=
 // c[s+1] in float arithmetic), c the running sum of w, b >= 0, and
@@ -16,6 +18,11 @@
 // the previous one, in IEEE arithmetic too, hence keys map to buckets in key
 // order and a partition by model buckets is a valid sample-sort partition:
 // the model only decides how balanced the buckets are, never the result.
+// The calibration evens out what the lines miss of the curve inside a cluster:
+// the cells of p are dealt to buckets by the sample's ranks, so a bucket's
+// share of the sample is right to about a cell.  (8 Gaussian clusters, 2^28
+// doubles: largest bucket 3.1 times the mean -> 1.6; the uncalibrated sizes
+// cost 0.1 ms in the next level and 0.2 ms in the leaves.)
 // A "heavy" key (one that repeats among the sample quantiles, as for the plain
 // splitters' equality buckets) splits its model bucket into below / equal /
 // above, and its equal bucket needs no sort.
@@ -60,10 +67,12 @@ constexpr int LR_LEAF_ITERS = 8;
 constexpr float LR_STEP = 0.02f;  // Adam step, relative to the parameters' scale
 constexpr float LR_TABLE_SEARCH_FRAC = 0.25f;
 
+constexpr int LR_CELLS = 4096;    // cells of p dealt to buckets by the calibration
+
 // A leaf: p = a + b * float(key - base) (0 below base), clamped to the
-// leaf's sample-CDF range [lo, hi].
+// leaf's sample-CDF range [lo, hi].  (Read as one 16-byte word and its rest.)
 template <typename K>
-struct LeafParam {
+struct alignas(16) LeafParam {
     K base;          // the leaf's first sample key
     float a, b;
     float lo, hi;
@@ -80,6 +89,8 @@ struct LearnedSet {
     LeafParam<K> leaf[LR_LEAVES];
     K heavy[NB];         // per model bucket: its heavy key (if flagged)
     uint16_t bid[NB];    // per model bucket: first bucket id | 0x100 if it has a heavy key
+    uint32_t calibrated; // cal gives the bucket (no heavy keys)
+    alignas(16) uint8_t cal[LR_CELLS];  // per cell of p: its bucket
     // bucket layout and diagnostics
     uint64_t region_off[NB];
     uint64_t region_cap[NB];
@@ -157,12 +168,18 @@ __device__ __forceinline__ uint32_t model_bucket(float p, uint32_t nmodel) {
     return (uint32_t)r > nmodel - 1 ? nmodel - 1 : (uint32_t)r;
 }
 
+__device__ __forceinline__ uint32_t cell_of(float p) {
+    const int c = (int)(p * (float)LR_CELLS);  // (p is in [0, 1])
+    return c < 0 ? 0u : (uint32_t)min(c, LR_CELLS - 1);
+}
+
 // bucket id of a key under a learned set held in shared memory
 template <typename K>
 __device__ __forceinline__ uint32_t learned_bucket(const LearnedSet<K>& L, K key) {
     const float p0 = root_p0<K>(L, key);
-    const LeafParam<K>& lp = L.leaf[leaf_of(p0)];
-    const uint32_t r = model_bucket(leaf_p<K>(lp, key), L.nmodel);
+    const float p = leaf_p<K>(L.leaf[leaf_of(p0)], key);
+    if (L.calibrated) return L.cal[cell_of(p)];
+    const uint32_t r = model_bucket(p, L.nmodel);
     const uint32_t e = L.bid[r];
     uint32_t id = e & 0xFFu;
     if (e >> 8) {
@@ -338,7 +355,7 @@ __global__ void __launch_bounds__(LR_THREADS) learned_root_kernel(const K* __res
     __syncthreads();
     bool fit = sd.count >= LR_MIN_KEYS;
     bool searches = false;
-    if (fit && !plain[sgi].direct) {  // (a direct table never searches, and its sample is not sorted)
+    if (fit && plain[sgi].route == ROUTE_SPLIT) {  // (the other routes never search, and their sample is not sorted)
         const SplitSet<K>& ps = plain[sgi];
         const SlotMap<K> fmap = ps.slot_map;
         uint32_t mine = 0;
@@ -581,6 +598,9 @@ __global__ void __launch_bounds__(NB) learned_finish_kernel(const K* __restrict_
     __shared__ uint32_t wt32[32];
     __shared__ uint64_t wt64[32];
     __shared__ uint32_t max_s, tot_ids_s, sorted_s;
+    __shared__ uint32_t cells[LR_CELLS];
+    __shared__ uint32_t rank0[NB + 1];
+    __shared__ uint8_t last[NB];
     __shared__ float loss_s, top_w[NB / 32];
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -627,6 +647,46 @@ __global__ void __launch_bounds__(NB) learned_finish_kernel(const K* __restrict_
     first_heavy[tid] = 0xFFFFFFFFu;
     const bool heavy = tid < (int)ps.nuniq && ((ps.eq_mask[tid >> 5] >> (tid & 31)) & 1u);
     const uint32_t nheavy = (uint32_t)__syncthreads_count(heavy);
+    const bool calibrated = nheavy == 0;
+    uint32_t cal_count = 0;  // samples of bucket tid
+    if (calibrated) {
+        // the sample's histogram over the cells of p, and each cell to the
+        // bucket that the middle of its samples falls in (in rank)
+        constexpr int PER = LR_CELLS / NB;  // cells per thread
+        static_assert(PER == 16, "a thread writes its cells' buckets as one 16-byte word");
+        for (int i = tid; i < LR_CELLS; i += NB) cells[i] = 0;
+        rank0[tid] = tid ? m : 0u;
+        if (tid == 0) rank0[NB] = m;
+        __syncthreads();
+        for (uint32_t i = tid; i < m; i += NB) {
+            const K x = smp[i];
+            atomicAdd(&cells[cell_of(leaf_p<K>(L.leaf[leaf_of(root_p0<K>(L, x))], x))], 1u);
+        }
+        __syncthreads();
+        uint32_t sum = 0;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) sum += cells[tid * PER + k];
+        uint32_t run = block_exclusive_scan_first<NB, uint32_t>(sum, wt32, (uint32_t*)nullptr);
+        const float per_rank = (float)nb / (float)(2 * m);  // (a monotone product: buckets rise with the cells)
+        uint32_t before[PER], bk[PER];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const uint32_t c = cells[tid * PER + k];
+            before[k] = run;
+            bk[k] = min((uint32_t)((float)(2 * run + c) * per_rank), (uint32_t)(nb - 1));
+            L.cal[tid * PER + k] = (uint8_t)bk[k];
+            run += c;
+        }
+        last[tid] = (uint8_t)bk[PER - 1];
+        __syncthreads();
+        uint32_t prev = tid ? last[tid - 1] : 0u;
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+            for (; prev < bk[k]; ++prev) rank0[prev + 1] = before[k];
+        __syncthreads();
+        cal_count = rank0[tid + 1] - rank0[tid];
+    }
+    if (tid == 0) L.calibrated = calibrated ? 1u : 0u;
     uint32_t nmodel = NB - 2 * nheavy;
     if (nmodel > (uint32_t)(2 * nb)) nmodel = 2 * nb;  // no more model buckets than the plain path aims for
     if (nmodel < 2) nmodel = 2;
@@ -646,10 +706,11 @@ __global__ void __launch_bounds__(NB) learned_finish_kernel(const K* __restrict_
     const uint32_t base_id = id < NB ? id : NB - 1;
     L.bid[tid] = (uint16_t)(base_id | (has_heavy ? 0x100u : 0u));
     if (tid == 0) {
-        L.nmodel = nmodel;
-        L.nbuckets = tot_ids_s;  // (the scan's total, written by one thread to shared memory)
+        L.nmodel = calibrated ? (uint32_t)nb : nmodel;
+        // (the scan's total, written by one thread to shared memory)
+        L.nbuckets = calibrated ? (uint32_t)nb : tot_ids_s;
     }
-    hist[tid] = 0;
+    hist[tid] = cal_count;
     __syncthreads();
 
     // the "equal" bucket of each heavy model bucket r is base_id[r] + 1
@@ -662,7 +723,8 @@ __global__ void __launch_bounds__(NB) learned_finish_kernel(const K* __restrict_
     // the sample through the model: its bucket histogram, and the balance of
     // the buckets that are sorted further (an equal bucket holds one key
     // value, however many times it repeats, and is only copied)
-    for (uint32_t i = tid; i < m; i += blockDim.x) atomicAdd(&hist[learned_bucket<K>(L, smp[i])], 1u);
+    if (!calibrated)
+        for (uint32_t i = tid; i < m; i += blockDim.x) atomicAdd(&hist[learned_bucket<K>(L, smp[i])], 1u);
     __syncthreads();
     const uint32_t c = hist[tid];
     if (c && !((L.bucket_eq[tid >> 5] >> (tid & 31)) & 1u)) {

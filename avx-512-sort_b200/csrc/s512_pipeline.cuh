@@ -2,6 +2,8 @@
 // (included by the translation units that sort: s512_sort.cu, s512_segsort.cu).
 #pragma once
 
+#include <algorithm>
+
 #include "s512_runtime.cuh"
 #include "s512_sortpipe.cuh"
 
@@ -9,7 +11,7 @@ namespace s512 {
 
 // Tile shapes of the partition kernel per key size: levels with many segments
 // (PartShape), and a level that is one whole array (PartShapeOne).  512
-// threads and 24-32 KB of keys per tile: two blocks (2 x ~90 KB of shared
+// threads and 24-32 KB of keys per tile: two blocks (2 x ~85-110 KB of shared
 // memory) share an SM.
 template <typename K> struct PartShape;
 template <> struct PartShape<uint32_t> { static constexpr int THREADS = 512, IPT = 12; };
@@ -113,15 +115,6 @@ static int sort_one_leaf(DevCtx& C, InCodec in, OutCodec out, uint32_t n, cudaSt
     }
 }
 
-// The partition kernel fetches tiles by bulk copy when every input array is
-// 16-byte aligned (segment and tile offsets keep that alignment).
-template <typename C>
-static bool codec_aligned(const C& c) {
-    for (int k = 0; k < C::NARR; ++k)
-        if (reinterpret_cast<uintptr_t>(c.arr(k)) & 15u) return false;
-    return true;
-}
-
 // ---------------------------------------------------------------------------
 // The first partition level of a host-pointer sort, fed while the caller's
 // page-locked arrays are still being copied in: the sample is read from the
@@ -155,13 +148,12 @@ struct Level {
     uint32_t ntiles_bound;
     K* out;
     uint64_t junk;              // offset in out of JUNK_KEYS keys past every region (overflow writes)
-    bool aligned;               // every tile starts 16-byte aligned (bulk copies allowed)
 };
 
 template <typename K, typename InCodec, typename UserOut, typename Shape = PartShape<K>>
 static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, size_t n, cudaStream_t st,
                      LevelCtl* ctl, LevelCtl* next_ctl_dev, SegDesc* next_segs, uint32_t next_cap,
-                     PhaseTimer& tm, s512_stats& S, LevelCtl* host_ctl, bool learned,
+                     PhaseTimer& tm, s512_stats& S, LevelCtl* host_ctl, bool learned, uint64_t max_seg,
                      const HostFeed* feed = nullptr) {
     constexpr int KB = sizeof(K);
     const uint32_t nsegs = L.nsegs;
@@ -178,8 +170,10 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
         if (!base) return S512_ERR_ALLOC;
         for (int c = 0; c <= NCLASS; ++c) items[c] = (LeafItem<K>*)(base + (size_t)c * item_cap * sizeof(LeafItem<K>));
     }
-    LearnedSet<K>* lsets = learned ? (LearnedSet<K>*)C.get("lsets", (size_t)nsegs * sizeof(LearnedSet<K>)) : nullptr;
-    if (!samples || !splits || !counts || (learned && !lsets)) return S512_ERR_ALLOC;
+    // (no segment worth a fit: the splitters route the level)
+    const bool fit = learned && (level == 0 || max_seg >= LR_MIN_KEYS);
+    LearnedSet<K>* lsets = fit ? (LearnedSet<K>*)C.get("lsets", (size_t)nsegs * sizeof(LearnedSet<K>)) : nullptr;
+    if (!samples || !splits || !counts || (fit && !lsets)) return S512_ERR_ALLOC;
 
     const int t0 = tm.mark();
     S512_CUDA_TRY(cudaMemsetAsync(ctl, 0, sizeof(LevelCtl), st));
@@ -195,12 +189,12 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
         S512_LAUNCH_CHECK();
         auto fn = split_kernel<K>;
         S512_CUDA_TRY(C.prepare((const void*)fn, split_smem<K>()));
-        fn<<<nsegs, SAMPLE_THREADS, split_smem<K>(), st>>>(samples, L.segs, splits, KB, learned ? 1 : 0);
+        fn<<<nsegs, SAMPLE_THREADS, split_smem<K>(), st>>>(samples, L.segs, splits, KB, fit ? 1 : 0);
         S512_LAUNCH_CHECK();
     }
     S.kernel_launches += 2;
     int tfit0 = -1;
-    if (learned) {
+    if (fit) {
         // the model is fitted to the same sorted sample; the split set above
         // stays as its fallback and supplies the heavy keys
         uint32_t* lfirst = (uint32_t*)C.get("lr_first", (size_t)nsegs * (LR_LEAVES + 1) * sizeof(uint32_t));
@@ -234,7 +228,6 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
     pa.tile_first = 0;
     pa.tile_counter = &ctl->tile_counter;
     pa.nsegs = nsegs;
-    pa.tma = (L.aligned && codec_aligned(L.in)) ? 1 : 0;
     pa.learned = lsets;
     pa.inject_timeout = (fault & S512_FAULT_TIMEOUT) ? 1 : 0;
     auto pfn = partition_kernel<K, InCodec, Shape::THREADS, Shape::IPT>;
@@ -253,8 +246,7 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
             pc.tile_first = c * tpc;
             pc.ntiles = (c + 1) * tpc < L.ntiles_host ? (c + 1) * tpc : L.ntiles_host;
             pc.tile_counter = cctr + c;
-            const uint32_t claims = (pc.ntiles - pc.tile_first + CLAIM_GROUP_ONE_SEG - 1) / CLAIM_GROUP_ONE_SEG;
-            const int g = pgrid < (int)claims ? pgrid : (int)claims;
+            const int g = std::min(pgrid, (int)(pc.ntiles - pc.tile_first));
             S512_CUDA_TRY(cudaStreamWaitEvent(st, feed->ready[c], 0));
             pfn<<<g, Shape::THREADS, psmem, st>>>(pc, L.in);
             S512_LAUNCH_CHECK();
@@ -344,7 +336,7 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
     const int t4 = tm.mark();
 
     if (lsets && host_ctl->learned_used) S.learned_levels += 1;
-    if (lsets) S.learned_rejected += host_ctl->plain_used;
+    if (learned) S.learned_rejected += host_ctl->plain_used;
     if (level < S512_MAX_LEVELS) {
         S.partition_keys[level] += (level == 0) ? (uint64_t)n : 0;
         S.partition_launches[level] += 1;
@@ -382,9 +374,7 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
 //
 // `whole` says that segs0 is one segment covering the caller's array from
 // element 0 with its tile fields set (sort_pipeline); any other list, even of
-// one segment, is laid out on the device (a lone segment of a batch starts
-// wherever the caller's segment starts, so its tiles need not be 16-byte
-// aligned for the bulk copy).
+// one segment, is laid out on the device.
 template <typename K, typename UserIn, typename UserOut>
 static int run_levels(DevCtx& C, UserIn uin, UserOut uout, SegDesc* segs0, uint32_t nsegs0, uint64_t keys0,
                       cudaStream_t st, PhaseTimer& tm, s512_stats& S, bool whole, bool learned = false,
@@ -425,7 +415,6 @@ static int run_levels(DevCtx& C, UserIn uin, UserOut uout, SegDesc* segs0, uint3
         L0.ntiles_host = (uint32_t)((keys0 + TILE_ONE - 1) / TILE_ONE);
         L0.ntiles_dev = nullptr;
         L0.ntiles_bound = L0.ntiles_host;
-        L0.aligned = true;
     } else {
         const uint32_t bound = (uint32_t)(keys0 / TILE) + nsegs0 + 1;
         uint32_t* tile_seg = (uint32_t*)C.get("tile_seg", (size_t)bound * sizeof(uint32_t));
@@ -440,14 +429,13 @@ static int run_levels(DevCtx& C, UserIn uin, UserOut uout, SegDesc* segs0, uint3
         L0.ntiles_host = 0;
         L0.ntiles_dev = &ctls[1].ntiles_next;
         L0.ntiles_bound = bound;
-        L0.aligned = false;  // segment starts are wherever the caller's segments start
     }
     if (!single) S512_TRY_RC(wait_feed(feed, st));  // (only a whole array is fed chunk by chunk)
     int rc = single ? run_level<K, UserIn, UserOut, PartShapeOne<K>>(C, L0, 0, uout, keys0, st, &ctls[0], &ctls[1],
                                                                       segbuf[1], next_cap, tm, S, host_ctl, learned,
-                                                                      feed)
+                                                                      keys0, feed)
                     : run_level<K, UserIn, UserOut>(C, L0, 0, uout, keys0, st, &ctls[0], &ctls[1], segbuf[1],
-                                                    next_cap, tm, S, host_ctl, learned);
+                                                    next_cap, tm, S, host_ctl, learned, keys0);
     if (rc) return rc;
     S.levels = 1;
 
@@ -489,10 +477,9 @@ static int run_levels(DevCtx& C, UserIn uin, UserOut uout, SegDesc* segs0, uint3
         Ln.ntiles_bound = ntiles_bound;
         Ln.out = out_buf;
         Ln.junk = need;
-        Ln.aligned = true;
         // the tile count lives in tctl, so the level's own control block is the other one
         rc = run_level<K, Raw<K>, UserOut>(C, Ln, level, uout, keys0, st, lctl, tctl, nxt, next_cap, tm, S,
-                                           host_ctl, learned);
+                                           host_ctl, learned, host_ctl->max_bucket);
         if (rc) return rc;
         if (level < S512_MAX_LEVELS) S.partition_keys[level] += next_keys;
         nsegs = host_ctl->n_next;

@@ -49,6 +49,9 @@ struct SegDesc {
     uint32_t ntiles;
 };
 
+// What finds the bucket of a segment's keys.
+enum : uint32_t { ROUTE_SPLIT = 0, ROUTE_LEARNED = 1, ROUTE_TABLE = 2, ROUTE_LINEAR = 3 };
+
 // Slot of a key in the direct table: its offset from lo, cut to 32 bits, times
 // a fixed-point factor.  fast() is right for keys in [lo, lo + range] and sets
 // `out` for any below lo or too far above; slot() is right for all (keys
@@ -111,9 +114,10 @@ struct SplitSet {
     K slot_hi;
     alignas(16) uint16_t slot_tab[SPLIT_SLOTS + 8];
     // A segment whose sample spreads over many slots is split at slot
-    // boundaries (direct): a key's bucket is then dir_tab[dir_map(key)], with
-    // no splitter left to compare (uniq holds the same boundaries as keys).
-    uint32_t direct;
+    // boundaries (route): a key's bucket is then dir_tab[dir_map(key)], or
+    // dir_map(key) itself where the sample is spread evenly, with no splitter
+    // left to compare (uniq holds the same boundaries as keys).
+    uint32_t route;      // ROUTE_*
     DirectMap<K> dir_map;
     alignas(16) uint8_t dir_tab[DIRECT_SLOTS];
 };
@@ -331,7 +335,7 @@ __device__ void make_splitters(Smp smp, uint32_t m, uint64_t count, int nb, Spli
         out->nbuckets = nbk;
         out->has_eq = w.total_eq ? 1u : 0u;
         out->nuniq = K_u;
-        out->direct = 0;
+        out->route = ROUTE_SPLIT;
     }
 }
 
@@ -351,8 +355,9 @@ __global__ void __launch_bounds__(NB) splitter_kernel(const K* __restrict__ samp
 
 // Split a segment at slot boundaries, from the histogram of its samples over
 // the slots: no sort, no splitter search, and the partition pass finds a key's
-// bucket with one table byte.  A slot goes to the bucket that the middle of
-// its samples falls in (in rank), so bucket ids rise with the slots.  Returns
+// bucket with one table byte, or none where the sample is spread evenly.  A
+// slot goes to the bucket that the middle of its samples falls in (in rank),
+// so bucket ids rise with the slots.  Returns
 // false, with nothing written, when the sample is not spread finely enough
 // over the slots: a slot that holds half a bucket's share (repeated values,
 // clusters) would leave uneven buckets and needs splitters between keys.
@@ -365,7 +370,9 @@ __device__ bool make_direct(const K (&key)[IPT], uint32_t m, uint64_t count, int
     struct Scratch {
         SplitScratch<K> w;
         uint32_t first_slot[NB + 1], rank0[NB + 1];  // per bucket: its first slot, the samples before it
+        uint32_t sumsq;
         uint8_t last[THREADS];                       // per thread: the bucket of its last slot
+        alignas(4) uint16_t before[DIRECT_SLOTS + 1];  // per slot: the samples before it
     };
     unsigned char* hist = smem;
     Scratch& d = *reinterpret_cast<Scratch*>(smem + DIRECT_SLOTS * sizeof(uint32_t));
@@ -436,32 +443,55 @@ __device__ bool make_direct(const K (&key)[IPT], uint32_t m, uint64_t count, int
             run += c[k];
         }
     }
-    uint32_t pack[PER / 4];
 #pragma unroll
-    for (int j = 0; j < PER / 4; ++j)
-        pack[j] = bk[4 * j] | (bk[4 * j + 1] << 8) | (bk[4 * j + 2] << 16) | (bk[4 * j + 3] << 24);
-    reinterpret_cast<uint4*>(out->dir_tab)[t] = make_uint4(pack[0], pack[1], pack[2], pack[3]);
+    for (int j = 0; j < PER / 2; ++j)
+        reinterpret_cast<uint32_t*>(d.before)[t * (PER / 2) + j] = rank[2 * j] | (rank[2 * j + 1] << 16);
+    if (t == 0) {
+        d.before[DIRECT_SLOTS] = (uint16_t)m;
+        d.sumsq = 0;
+    }
     d.last[t] = (uint8_t)bk[PER - 1];
     __syncthreads();
-    uint32_t prev = t ? d.last[t - 1] : 0u;
-    if (t == 0) {
-        d.first_slot[0] = 0;
-        d.rank0[0] = 0;
+    // Evenly spread?  Then nb equal slots need no table, and their sizes do
+    // not carry the noise of the sample.  (Their sample counts are read off at
+    // the nearest of the fine slots.)  Even: the counts' squared deviation is
+    // about what chance gives (one share per bucket), and none stands out.
+    auto fine = [&](uint32_t j) { return (j * (uint32_t)DIRECT_SLOTS + (uint32_t)nb - 1) / (uint32_t)nb; };
+    uint32_t cl = 0;
+    if (t < (unsigned)nb) cl = (uint32_t)d.before[fine(t + 1)] - (uint32_t)d.before[fine(t)];
+    if (t < NB) {
+        const uint32_t sq = __reduce_add_sync(0xFFFFFFFFu, cl * cl);
+        if (lane == 0) atomicAdd(&d.sumsq, sq);
     }
+    const float share = (float)m / (float)nb;
+    const bool stands_out = __syncthreads_or((float)cl > 1.6f * share);
+    const bool linear = !stands_out && (float)d.sumsq / share - (float)m <= 1.4f * (float)nb + 6.0f;
+    if (linear) {
+        dm.mul = make_slot_map_fast<K>(lo, range, (uint32_t)nb).mul;
+    } else {
+        uint32_t pack[PER / 4];
 #pragma unroll
-    for (int k = 0; k < PER; ++k) {
-        for (; prev < bk[k]; ++prev) {
-            d.first_slot[prev + 1] = t * PER + k;
-            d.rank0[prev + 1] = rank[k];
+        for (int j = 0; j < PER / 4; ++j)
+            pack[j] = bk[4 * j] | (bk[4 * j + 1] << 8) | (bk[4 * j + 2] << 16) | (bk[4 * j + 3] << 24);
+        reinterpret_cast<uint4*>(out->dir_tab)[t] = make_uint4(pack[0], pack[1], pack[2], pack[3]);
+        uint32_t prev = t ? d.last[t - 1] : 0u;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            for (; prev < bk[k]; ++prev) {
+                d.first_slot[prev + 1] = t * PER + k;
+                d.rank0[prev + 1] = rank[k];
+            }
         }
+        if (t == 0) d.rank0[0] = 0;
     }
     __syncthreads();
     if (t < NB) {
         const bool live = t < (unsigned)nb;
-        d.w.cap[t] = live ? bucket_cap(d.rank0[t + 1] - d.rank0[t], (double)count / (double)m, count) : 0ull;
+        const uint32_t c = linear ? cl : d.rank0[t + 1] - d.rank0[t];
+        d.w.cap[t] = live ? bucket_cap(c, (double)count / (double)m, count) : 0ull;
         // splitter t: the last key before bucket t + 1 (slot 0 is always in
         // bucket 0: it holds less than half a bucket's samples)
-        const uint32_t s = t + 1 < (unsigned)nb ? d.first_slot[t + 1] : (uint32_t)DIRECT_SLOTS;
+        const uint32_t s = t + 1 >= (unsigned)nb ? 0xFFFFFFFFu : linear ? t + 1 : d.first_slot[t + 1];
         d.w.uniq[t] = s <= dm.slot(lo + range) ? dm.first_key(s) - 1 : KeyMax<K>::value;
         out->range_b[t] = live ? (uint8_t)t : (uint8_t)0;
         out->eq_b[t] = 0;
@@ -472,7 +502,7 @@ __device__ bool make_direct(const K (&key)[IPT], uint32_t m, uint64_t count, int
         out->nbuckets = (uint32_t)nb;
         out->has_eq = 0;
         out->nuniq = (uint32_t)nb - 1;
-        out->direct = 1;
+        out->route = linear ? ROUTE_LINEAR : ROUTE_TABLE;
         out->dir_map = dm;
     }
     return true;
@@ -611,36 +641,47 @@ namespace s512 {
 // ===========================================================================
 // 4. The partition pass (persistent; tiles claimed in runs)
 //
-// What bounds it: issue slots and the shared-memory pipe (wavefronts), not HBM,
-// so the classification is kept short: a segment split at slot boundaries
-// (ROUTE_DIRECT) needs a subtraction, a shift, a multiply and one table byte
-// per key.  One 256-way pass over 2^28 doubles: 1.58 ms when every key was
-// clamped, looked up and compared with the splitters of its slot, 1.25 ms
-// (level 0) and 1.64 -> 1.38 ms (level 1) direct; the floor is 0.66 ms.
+// Every tile of keys is classified, ranked within its bucket by shared-memory
+// atomics, put in its bucket's bin in shared memory and written out from
+// there, a group of lanes per bin.  Where a tile's keys of bucket b go inside
+// the bucket's region is reserved with one global atomic add per (tile,
+// bucket) on the segment's fill counter of b: the pass is not stable (a
+// bucket's keys land in the order their tiles reserved, and the leaves sort
+// them anyway), so no tile ever waits for another and tiles may be processed
+// in any order.  The counters end as the bucket sizes.  A reservation past the
+// region's capacity (the sample's 6-sigma bound) drops the tile's keys of that
+// bucket and reports an overflow; the level is then redone with exact counts.
 //
-// Every tile of keys is classified, ranked within the tile by shared-memory
-// atomics, staged in bucket order in shared memory and written out with
-// coalesced stores.  Where a tile's keys of bucket b go inside the bucket's
-// region is reserved with one global atomic add per (tile, bucket) on the
-// segment's fill counter of b: the pass is not stable (a bucket's keys land in
-// the order their tiles reserved, and the leaves sort them anyway), so no
-// tile ever waits for another and tiles may be processed in any order.  The
-// counters end as the bucket sizes.  A reservation past the region's
-// capacity (the sample's 6-sigma bound) drops the tile's keys of that bucket
-// and reports an overflow; the level is then redone with exact counts.
+// What bounds it is the shared-memory pipe (wavefronts per key), then issue
+// slots; HBM is third.  So a key costs one random shared access for its bucket
+// (none on ROUTE_LINEAR), one atomic for its rank and one store into its bin:
+// a bin holds a fixed number of keys, about 2.5 times a bucket's share of the
+// tile, so its place needs no scan and no lookup, and the write-out reads a
+// bin's pointer and count once per group of lanes instead of a bucket id and a
+// pointer per key.  A tile with a fuller bucket (sorted or skewed input) is
+// staged compactly in bucket order instead, with a scan of the counts and a
+// bucket id per key.
 //
-// Pipeline per block: the next tile travels into the second shared-memory
-// buffer by a 1-D bulk copy (TMA, completing on an mbarrier) while the
-// current one is ranked, staged and written; the buffer that held a tile's
-// raw keys is reused to stage them in bucket order.  Three block barriers per
-// tile: histogram complete | bucket starts known | staging complete.  Two
-// blocks share an SM, so one block's barrier phases overlap the other's
-// memory traffic.  When an input array is not 16-byte aligned the tiles are
-// read with plain loads instead (a.tma == 0).
+// The next tile's keys are loaded into registers as soon as the current ones
+// are in their bins, a run of 512 * 8 bytes per load instruction of the block;
+// the loads complete while the tile is reserved and written.  Three block
+// barriers per tile: bins free | bins filled | places known; a warp that has
+// written its bins classifies its next keys before it waits.  Two blocks share
+// an SM, so one block's barrier phases overlap the other's memory traffic.
+// (Loads must stay raw bits until then: encoding them where they are loaded
+// made every thread wait there.  Bulk copies into shared memory, which this
+// pass used before, cost two more shared wavefronts per 32 keys.)
+// Measured, one pass over 2^28 doubles, floor 0.66 ms: level 0 (ROUTE_TABLE)
+// 1.25 -> 1.20 ms, level 1 (ROUTE_LINEAR) 1.38 -> 1.17 ms; 1.58 and 1.64 ms
+// when every key was clamped, compared with the splitters of its slot and
+// staged with a bucket id.  2^20 int32: 29 -> 7.5 us (shorter claim runs).
 constexpr int SEG_SMEM = 256;  // segment tables up to this size are searched in shared memory
-// Consecutive tiles a block claims at once: one segment's tables are loaded
-// once per group, so levels with many segments take longer runs; a single
-// segment takes short ones (a finer split of the last tiles among blocks).
+// Consecutive tiles a block claims at once, at most: one segment's tables are
+// loaded once per group, so levels with many segments take longer runs; a
+// single segment takes short ones (a finer split of the last tiles among
+// blocks).  A launch of few tiles takes shorter runs still, so that every
+// block has some: 733 tiles of one segment 73 -> 31 us, 171 of 2^20 int32 37 -> 7.5 us
+// against runs of 4 with two claimed at once.
 constexpr uint32_t CLAIM_GROUP_ONE_SEG = 4;
 constexpr uint32_t CLAIM_GROUP_MANY_SEGS = 16;
 // Keys past the regions of a level buffer where a bucket that overflowed its
@@ -662,7 +703,6 @@ struct PartArgs {
     const uint32_t* ntiles_dev;   // tile count written by prepare_level_kernel
     uint32_t tile_first;          // first tile of the launch (a level fed in chunks launches per chunk)
     uint32_t* tile_counter;       // the launch's claim counter (zeroed)
-    int tma;                      // tiles arrive by bulk copy
     const LearnedSet<K>* learned; // per segment learned model (nullptr: splitters only)
     int inject_timeout;           // testing: tile 1 waits, with a short bound, on a flag nothing sets
 };
@@ -686,29 +726,53 @@ struct DirectTables {
     alignas(16) uint8_t tab[DIRECT_SLOTS];
 };
 
-// What finds the bucket of a segment's keys.
-enum : uint32_t { ROUTE_SPLIT = 0, ROUTE_LEARNED = 1, ROUTE_DIRECT = 2 };
-
 // Bytes of a LearnedSet that inference reads (its leading fields).
 template <typename K>
 constexpr size_t learned_model_bytes() { return offsetof(LearnedSet<K>, region_off); }
 
+// Keys a bin holds: about 2.5 times the even share of a tile (16 keys of 64
+// bits, 24 of 32 bits), so that on evenly split keys a fuller one is rare (a
+// bucket at 1.4 times its share overflows one tile in thousands) and two
+// blocks fit an SM.  Odd, so that equal places of different bins, which fill
+// at the same time, lie on different banks.
+__host__ __device__ constexpr int bin_cap(int tile) { return (tile * 5 / 2 / NB) | 1; }
+// A segment's tiles use the bins where that makes an average bin half full at
+// most, and where places in its regions fit 32 bits.
+__host__ __device__ constexpr bool use_bins(int tile, uint32_t nbuckets, uint64_t seg_count) {
+    return (uint32_t)tile * 2 <= nbuckets * (uint32_t)bin_cap(tile) && seg_count < (1ull << 31);
+}
+
 template <typename K, int THREADS, int IPT>
 struct PartSmem {
     static constexpr int TILE = THREADS * IPT;
-    alignas(128) unsigned char buf[2][TILE * sizeof(K)];
-    uint8_t bkt[TILE];
+    static constexpr int CAP = bin_cap(TILE);
+    struct Compact {
+        K stage[TILE];
+        uint8_t bkt[TILE];
+    };
+    union {
+        alignas(16) K bins[NB * CAP];
+        Compact c;
+    } u;
+    struct alignas(8) Bin {
+        uint32_t place, count;    // where the bin's key 0 goes in the segment's regions, and its keys
+    };
+    union {
+        Bin bin[NB];
+        uint64_t ptr[NB];         // compact tiles: where the bucket would put the tile's position 0
+    } w;
     uint64_t region_off[NB];
     uint64_t region_cap[NB];
-    uint64_t gptr[NB];            // bucket b's keys of the tile: position p goes to (K*)gptr[b] + p
-    uint32_t hist[NB];
-    uint32_t loc[NB];
+    alignas(16) uint32_t hist[NB];
+    alignas(16) uint32_t loc[NB];
     uint32_t seg_tile_start[SEG_SMEM];
-    uint64_t mbar[2];
-    uint32_t tile_cur, has_eq, route, abort;
-    SegDesc sd;                   // segment of the tile being processed
-    SegDesc iss_sd;               // thread 0: segment of the last tile it fetched
-    uint32_t iss_seg;
+    struct Tile {
+        uint64_t first;           // its first key in the input
+        uint32_t count;           // its keys (0: no more tiles)
+        uint32_t seg, index, pad_;
+    } tile[2];
+    uint64_t out_base;
+    uint32_t has_eq, route, bins;
     // a segment routes by one of these
     union {
         PlainTables<K> P;
@@ -723,23 +787,17 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) partition_kernel(Part
     using SM = PartSmem<K, THREADS, IPT>;
     SM& sm = *reinterpret_cast<SM*>(smem_part);
     constexpr int TILE = THREADS * IPT;
-    constexpr int ESZ = InCodec::ESZ;
-    constexpr int NARR = InCodec::NARR;
+    constexpr uint32_t CAP = SM::CAP;
     static_assert(TILE < (1 << 21), "rank and bucket share a 32-bit word");
     static_assert(TILE <= (int)JUNK_KEYS, "an overflowed bucket's keys of a tile fit the overflow area");
+    static_assert(sizeof(typename SM::Compact) <= sizeof(K) * NB * CAP, "the compact stage fits the bins' space");
+    static_assert(THREADS >= NB, "a thread per bucket");
     const int tid = threadIdx.x;
     const uint32_t ntiles = a.ntiles_dev ? *a.ntiles_dev : a.ntiles;
     const bool small_tab = a.tile_seg && a.nsegs <= (uint32_t)SEG_SMEM;
-    uint32_t cached_seg = 0xFFFFFFFFu;
+    const bool claimer = tid == THREADS - 1;  // (the last warp: the first ones reserve and scan)
 
-    if (tid == 0) {
-        mbar_init(&sm.mbar[0], 1);
-        mbar_init(&sm.mbar[1], 1);
-        fence_mbar_init();
-        sm.abort = 0;
-        sm.iss_seg = 0xFFFFFFFFu;
-    }
-    for (int b = tid; b < NB; b += THREADS) sm.hist[b] = 0;
+    if (tid < NB) sm.hist[tid] = 0;
     if (small_tab)
         for (uint32_t i = tid; i < a.nsegs; i += THREADS) sm.seg_tile_start[i] = a.segs[i].tile_start;
     __syncthreads();
@@ -754,183 +812,156 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) partition_kernel(Part
         }
         return lo;
     };
-    // thread 0: start the bulk copy of tile t into buffer b
-    auto issue = [&](uint32_t t, int b) {
-        const uint32_t seg = seg_of(t);
-        if (seg != sm.iss_seg) {  // (tiles come in runs of one segment)
-            sm.iss_sd = a.segs[seg];
-            sm.iss_seg = seg;
-        }
-        const SegDesc sd = sm.iss_sd;
-        const uint32_t ti = t - sd.tile_start;
-        const uint64_t first = sd.in_off + (uint64_t)ti * TILE;
-        const uint64_t rem = sd.count - (uint64_t)ti * TILE;
-        const uint32_t cnt = rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
-        const uint32_t bytes = (cnt * ESZ) & ~15u;
-        fence_proxy_async_smem();
-        mbar_arrive_expect_tx(&sm.mbar[b], bytes * NARR);
-        if (bytes) {
-#pragma unroll
-            for (int k = 0; k < NARR; ++k)
-                bulk_g2s(sm.buf[b] + (size_t)k * TILE * ESZ,
-                         static_cast<const unsigned char*>(in.arr(k)) + first * ESZ, bytes, &sm.mbar[b]);
-        }
-    };
-
-    // thread 0 claims claim_group consecutive tiles at a time, so that a block
-    // works through a run of one segment before it loads another's tables
-    const uint32_t claim_group = a.nsegs > 1 ? CLAIM_GROUP_MANY_SEGS : CLAIM_GROUP_ONE_SEG;
-    uint32_t grp_next = 0, grp_end = 0;
-    auto claim = [&]() -> uint32_t {
+    // The claimer takes claim_group consecutive tiles at a time: the first
+    // group by the block's index, the others from the counter.  A group is
+    // claimed with the last tile of the one before (the atomic's latency
+    // passes while that tile is processed).
+    const uint32_t most = a.nsegs > 1 ? CLAIM_GROUP_MANY_SEGS : CLAIM_GROUP_ONE_SEG;
+    const uint32_t claim_group = min(max((ntiles - min(a.tile_first, ntiles)) / (gridDim.x * 2), 1u), most);
+    uint32_t grp_next = a.tile_first + blockIdx.x * claim_group, grp_end = grp_next + claim_group, grp_ahead = 0;
+    uint32_t c_seg = 0xFFFFFFFFu, c_tile0 = 0;
+    uint64_t c_off = 0, c_count = 0;
+    auto next_tile = [&](typename SM::Tile* slot) {
         if (grp_next == grp_end) {
-            grp_next = a.tile_first + atomicAdd(a.tile_counter, claim_group);
+            grp_next = grp_ahead;
             grp_end = grp_next + claim_group;
         }
-        return grp_next++;
+        const uint32_t t = grp_next++;
+        if (grp_next == grp_end)
+            grp_ahead = a.tile_first + gridDim.x * claim_group + atomicAdd(a.tile_counter, claim_group);
+        slot->count = 0;
+        if (t >= ntiles) return;
+        const uint32_t seg = seg_of(t);
+        if (seg != c_seg) {  // (tiles come in runs of one segment)
+            c_seg = seg;
+            c_off = a.segs[seg].in_off;
+            c_count = a.segs[seg].count;
+            c_tile0 = a.segs[seg].tile_start;
+        }
+        const uint64_t at = (uint64_t)(t - c_tile0) * TILE;
+        slot->first = c_off + at;
+        slot->count = c_count - at < (uint64_t)TILE ? (uint32_t)(c_count - at) : (uint32_t)TILE;
+        slot->seg = seg;
+        slot->index = t;
     };
-    uint32_t t_next = 0;  // thread 0: the tile after the current one
-    if (tid == 0) {
-        const uint32_t t0 = claim();
-        sm.tile_cur = t0;
-        if (a.tma && t0 < ntiles) issue(t0, 0);
-        t_next = claim();
+    if (claimer) {
+        next_tile(&sm.tile[0]);
+        next_tile(&sm.tile[1]);
     }
     __syncthreads();
-    uint32_t phases = 0;  // bit b: the parity to wait for on buffer b's mbarrier
-    int b = 0;
 
-    while (true) {
-        // tile_cur is rewritten by thread 0 only after the first barrier of
-        // the iteration, and read again after the last one
-        const uint32_t t = sm.tile_cur;
-        if (t >= ntiles || sm.abort) break;
-        const uint32_t seg = seg_of(t);
-        const bool new_seg = seg != cached_seg;
-        if (new_seg) {
-            // the segment's descriptor and tables, read once per run of its
-            // tiles (the previous tile's write-out reads none of them)
-            if (tid < (int)(sizeof(SegDesc) / 4))
-                reinterpret_cast<uint32_t*>(&sm.sd)[tid] = reinterpret_cast<const uint32_t*>(&a.segs[seg])[tid];
-            const uint32_t route = a.learned && a.learned[seg].ok ? ROUTE_LEARNED
-                                   : a.splits[seg].direct         ? ROUTE_DIRECT
-                                                                  : ROUTE_SPLIT;
-            if (route == ROUTE_DIRECT) {
-                const SplitSet<K>& ss = a.splits[seg];
-                for (int i = tid; i < NB; i += THREADS) {
-                    sm.region_off[i] = ss.region_off[i];
-                    sm.region_cap[i] = ss.region_cap[i];
-                }
+    K key[IPT];  // the tile's keys, striped (element r*THREADS + tid); as stored until they are classified
+    auto load = [&](uint64_t first, uint32_t cnt) {
+        if (cnt == (uint32_t)TILE) {
+#pragma unroll
+            for (int r = 0; r < IPT; ++r) key[r] = in.raw(first + (uint32_t)(r * THREADS + tid));
+        } else {
+#pragma unroll
+            for (int r = 0; r < IPT; ++r)
+                if ((uint32_t)(r * THREADS + tid) < cnt) key[r] = in.raw(first + (uint32_t)(r * THREADS + tid));
+        }
+    };
+    uint32_t cnt = sm.tile[0].count, seg = sm.tile[0].seg, index = sm.tile[0].index;
+    load(sm.tile[0].first, cnt);
+    uint32_t cached_seg = 0xFFFFFFFFu;
+
+    for (uint32_t turn = 1; cnt != 0; turn ^= 1) {  // turn: the slot of the next tile
+        if (seg != cached_seg) {
+            // the segment's tables, read once per run of its tiles (the
+            // previous tile's write-out reads none of them)
+            const uint32_t route = a.learned && a.learned[seg].ok ? ROUTE_LEARNED : a.splits[seg].route;
+            const SplitSet<K>& ss = a.splits[seg];
+            const uint64_t* off = route == ROUTE_LEARNED ? a.learned[seg].region_off : ss.region_off;
+            const uint64_t* cap = route == ROUTE_LEARNED ? a.learned[seg].region_cap : ss.region_cap;
+            if (tid < NB) {
+                sm.region_off[tid] = off[tid];
+                sm.region_cap[tid] = cap[tid];
+            }
+            if (route == ROUTE_TABLE) {
                 const uint4* src = reinterpret_cast<const uint4*>(ss.dir_tab);
                 uint4* dst = reinterpret_cast<uint4*>(sm.T.D.tab);
                 for (int i = tid; i < DIRECT_SLOTS / 16; i += THREADS) dst[i] = src[i];
-                if (tid == 0) sm.T.D.map = ss.dir_map;
             } else if (route == ROUTE_LEARNED) {
-                const LearnedSet<K>& ls = a.learned[seg];
-                const uint32_t* src = reinterpret_cast<const uint32_t*>(&ls);
+                const uint32_t* src = reinterpret_cast<const uint32_t*>(&a.learned[seg]);
                 uint32_t* dst = reinterpret_cast<uint32_t*>(sm.T.model);
                 for (uint32_t i = tid; i < learned_model_bytes<K>() / 4; i += THREADS) dst[i] = src[i];
-                for (int i = tid; i < NB; i += THREADS) {
-                    sm.region_off[i] = ls.region_off[i];
-                    sm.region_cap[i] = ls.region_cap[i];
-                }
-            } else {
-                const SplitSet<K>& ss = a.splits[seg];
-                for (int i = tid; i < NB; i += THREADS) {
-                    sm.T.P.uniq[i] = ss.uniq[i];
-                    sm.region_off[i] = ss.region_off[i];
-                    sm.region_cap[i] = ss.region_cap[i];
-                    sm.T.P.range_b[i] = ss.range_b[i];
-                    sm.T.P.eq_b[i] = ss.eq_b[i];
+            } else if (route == ROUTE_SPLIT) {
+                if (tid < NB) {
+                    sm.T.P.uniq[tid] = ss.uniq[tid];
+                    sm.T.P.range_b[tid] = ss.range_b[tid];
+                    sm.T.P.eq_b[tid] = ss.eq_b[tid];
                 }
                 if (tid < NB / 32) sm.T.P.eq_mask[tid] = ss.eq_mask[tid];
-                {
-                    const uint4* src = reinterpret_cast<const uint4*>(ss.slot_tab);
-                    uint4* dst = reinterpret_cast<uint4*>(sm.T.P.tab);
-                    for (int i = tid; i < (SPLIT_SLOTS + 8) * 2 / 16; i += THREADS) dst[i] = src[i];
-                }
-                if (tid == 0) {
+                const uint4* src = reinterpret_cast<const uint4*>(ss.slot_tab);
+                uint4* dst = reinterpret_cast<uint4*>(sm.T.P.tab);
+                for (int i = tid; i < (SPLIT_SLOTS + 8) * 2 / 16; i += THREADS) dst[i] = src[i];
+            }
+            if (tid == 0) {
+                sm.out_base = a.segs[seg].out_base;
+                sm.route = route;
+                sm.bins = use_bins(TILE, route == ROUTE_LEARNED ? a.learned[seg].nbuckets : ss.nbuckets,
+                                   a.segs[seg].count);
+                if (route == ROUTE_TABLE || route == ROUTE_LINEAR) {
+                    sm.T.D.map = ss.dir_map;
+                } else if (route == ROUTE_SPLIT) {
                     sm.has_eq = ss.has_eq;
                     sm.T.P.fmap = ss.slot_map;
                     sm.T.P.fhi = ss.slot_hi;
                 }
             }
-            if (tid == 0) sm.route = route;
             cached_seg = seg;
+            __syncthreads();
         }
-        bool data_ok = true;
-        if (a.tma) {
-            // every thread waits on the barrier itself: the bulk copy's data is
-            // then visible to it without a block barrier
-            data_ok = mbar_wait_bounded(&sm.mbar[b], (phases >> b) & 1u);
-            phases ^= 1u << b;
-            if (!data_ok) raise_error(&a.ctl->err, DEV_ERR_TIMEOUT);
-        }
-        if (a.inject_timeout && t == 1) {
+        if (a.inject_timeout && index == 1) {
             // injected failure: a wait on a flag that nothing sets, with a
-            // short bound; the tile then gives up and writes nothing
+            // short bound; the block then gives up and writes nothing more
             uint32_t spins = 0;
             while (!*(volatile uint32_t*)&a.ctl->never_set && ++spins < 1024u) __nanosleep(100);
-            data_ok = false;
             raise_error(&a.ctl->err, DEV_ERR_TIMEOUT);
+            break;
         }
-        if (new_seg) __syncthreads();  // the segment's descriptor and tables in shared memory
-        // (the descriptor stays in shared memory: registers hold the keys)
-        const uint32_t ti = t - sm.sd.tile_start;
-        const uint64_t base = sm.sd.in_off + (uint64_t)ti * TILE;
-        const uint64_t rem = sm.sd.count - (uint64_t)ti * TILE;
-        const uint32_t cnt = rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
-        const uint32_t tma_elems = a.tma ? ((cnt * ESZ) & ~15u) / ESZ : 0u;
-        const uint32_t route = sm.route;
 
-        // a whole tile from the bulk copy (no per-key range checks)
-        const bool FULL = cnt == (uint32_t)TILE && tma_elems == (uint32_t)TILE;
-        {
-            // A. keys (striped: element r*THREADS + tid, from the bulk-copied
-            // tile; tail elements past the copied bytes from global memory),
-            // their buckets and their ranks within the tile
-            K key[IPT];
-            uint32_t br[IPT];  // 4 * bucket | rank << 11
+        // A. buckets and ranks.  All IPT bucket lookups first: they are
+        // independent chains, so the scheduler can overlap them.
+        uint32_t br[IPT];  // 4 * bucket | rank << 11
+        bool over = !sm.bins;  // some bucket has more keys of the tile than a bin holds
+        auto classify = [&](auto full) {
+            constexpr bool FULL = decltype(full)::value;
+            const uint32_t route = sm.route;
 #pragma unroll
-            for (int r = 0; r < IPT; ++r) {
-                const uint32_t idx = (uint32_t)(r * THREADS + tid);
-                if (FULL) key[r] = in.decode(sm.buf[b], idx, TILE);
-                else if (idx < cnt) key[r] = idx < tma_elems ? in.decode(sm.buf[b], idx, TILE) : in.load(base + idx);
-            }
-            // all IPT bucket lookups first: they are independent chains of
-            // shared loads, so the scheduler can overlap them.  (Lanes past
-            // the end look up stale register contents, in bounds, and then
-            // carry the out-of-range bucket NB.)
-            if (route == ROUTE_DIRECT) {
+            for (int r = 0; r < IPT; ++r) key[r] = InCodec::enc(key[r]);
+            if (route >= ROUTE_TABLE) {
                 const DirectMap<K> dm = sm.T.D.map;
                 bool out = false;
+                // (lanes past the end look up stale register contents, in
+                // bounds, and then carry the out-of-range bucket NB)
 #pragma unroll
                 for (int r = 0; r < IPT; ++r) br[r] = dm.fast(key[r], out);
                 if (out) {  // a key outside the sample's range (2 in 16384 or so)
 #pragma unroll
                     for (int r = 0; r < IPT; ++r) br[r] = dm.slot(key[r]);
                 }
+                if (route == ROUTE_TABLE) {
 #pragma unroll
-                for (int r = 0; r < IPT; ++r) br[r] = (uint32_t)sm.T.D.tab[br[r]] << 2;
+                    for (int r = 0; r < IPT; ++r) br[r] = sm.T.D.tab[br[r]];
+                }
+#pragma unroll
+                for (int r = 0; r < IPT; ++r) br[r] <<= 2;
             } else if (route == ROUTE_LEARNED) {
 #pragma unroll
-                for (int r = 0; r < IPT; ++r) {
-                    const uint32_t idx = (uint32_t)(r * THREADS + tid);
-                    // (only the model prefix of the LearnedSet is in shared memory)
-                    if (FULL || idx < cnt)
+                for (int r = 0; r < IPT; ++r)  // (only the model prefix of the LearnedSet is in shared memory)
+                    if (FULL || (uint32_t)(r * THREADS + tid) < cnt)
                         br[r] = learned_bucket<K>(*reinterpret_cast<const LearnedSet<K>*>(sm.T.model), key[r]) << 2;
-                }
             } else {
                 const bool has_eq = sm.has_eq != 0;
                 const SlotRegs<K> fm(sm.T.P.fmap, sm.T.P.fhi);
 #pragma unroll
                 for (int r = 0; r < IPT; ++r) br[r] = sm.T.P.tab[fm(key[r])];  // slot entries first
 #pragma unroll
-                for (int r = 0; r < IPT; ++r) {
-                    const uint32_t idx = (uint32_t)(r * THREADS + tid);
-                    if (FULL || idx < cnt)
+                for (int r = 0; r < IPT; ++r)
+                    if (FULL || (uint32_t)(r * THREADS + tid) < cnt)
                         br[r] = bucket_from_slot<K>(br[r], key[r], has_eq, sm.T.P.uniq, sm.T.P.range_b, sm.T.P.eq_b,
                                                     sm.T.P.eq_mask) << 2;
-                }
             }
             if (!FULL) {
 #pragma unroll
@@ -958,22 +989,81 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) partition_kernel(Part
                         rank = atomicAdd(hist(br[r]), 1u);
                     }
                     br[r] |= rank << 11;
+                    over |= rank >= CAP;
                 }
             } else {
 #pragma unroll
                 for (int r = 0; r < IPT; ++r)
-                    if (FULL || br[r] < 4u * NB) br[r] |= atomicAdd(hist(br[r]), 1u) << 11;
+                    if (FULL || br[r] < 4u * NB) {
+                        br[r] |= atomicAdd(hist(br[r]), 1u) << 11;
+                        over |= br[r] >= (CAP << 11);
+                    }
             }
-            __syncthreads();  // (1) the tile's histogram is complete; the previous tile is written
+        };
+        if (cnt == (uint32_t)TILE) classify(std::true_type{});
+        else classify(std::false_type{});
+        __syncthreads();  // (1) the bins are free: the previous tile is written
 
-            // B. reserve the tile's share of each bucket's region, and the
-            // buckets' starts within the tile (exclusive scan by warp 0)
-            uint32_t h = 0;
-            unsigned long long off = 0;
-            if (tid < NB) {
-                h = sm.hist[tid];
-                if (h) off = atomicAdd(&a.fill[(size_t)seg * NB + tid], (unsigned long long)h);
+        // B. the keys into their buckets' bins
+        if (sm.bins) {
+#pragma unroll
+            for (int r = 0; r < IPT; ++r) {
+                const uint32_t b4 = br[r] & 0x7FFu, rank = br[r] >> 11;
+                if (b4 < 4u * NB && rank < CAP) sm.u.bins[(b4 >> 2) * CAP + rank] = key[r];
             }
+        }
+        const bool compact = __syncthreads_or(over);  // (2) bins and counts are complete
+
+        // C. reserve the tile's share of each bucket's region
+        uint32_t h = 0;
+        unsigned long long off = 0;
+        if (tid < NB) {
+            h = sm.hist[tid];
+            if (h) off = atomicAdd(&a.fill[(size_t)seg * NB + tid], (unsigned long long)h);
+        }
+        const uint32_t tile_cnt = cnt;
+        auto advance = [&]() {  // the next tile's keys (the current ones are staged)
+            const typename SM::Tile& nx = sm.tile[turn];
+            cnt = nx.count;
+            seg = nx.seg;
+            index = nx.index;
+            load(nx.first, cnt);
+        };
+        // where the bucket's keys of the tile go (an overflowed bucket's to the
+        // overflow area past the regions: the level is redone)
+        auto overflows = [&]() {
+            const bool ovf = off + h > sm.region_cap[tid];
+            if (ovf && h) raise_error(&a.ctl->err, DEV_ERR_OVERFLOW);
+            return ovf;
+        };
+        if (!compact) {
+            if (tid < NB) sm.hist[tid] = 0;
+            advance();
+            if (claimer) next_tile(&sm.tile[turn ^ 1]);
+            if (tid < NB) {
+                // (places fit 32 bits; an overflowed bucket is not written)
+                typename SM::Bin o;
+                o.place = (uint32_t)(sm.region_off[tid] + off);
+                o.count = overflows() ? 0u : h;
+                sm.w.bin[tid] = o;
+            }
+            K* const seg_out = a.out + sm.out_base;
+            __syncthreads();  // (3) places known
+            // D. each group of lanes writes out its bins
+            constexpr int GL = sizeof(K) == 8 ? 16 : 32, NG = THREADS / GL;
+            const uint32_t g = (uint32_t)tid / GL, l = (uint32_t)tid % GL;
+#pragma unroll 4
+            for (uint32_t b = g; b < (uint32_t)NB; b += NG) {
+                const typename SM::Bin o = sm.w.bin[b];
+                const K* src = sm.u.bins + b * CAP;
+                K* dst = seg_out + o.place;
+                if (l < o.count) dst[l] = src[l];
+                if (l + GL < o.count) dst[l + GL] = src[l + GL];
+                if (2 * GL < CAP && l + 2 * GL < o.count) dst[l + 2 * GL] = src[l + 2 * GL];
+            }
+            static_assert(CAP <= 3 * GL, "a bin is at most three keys per lane");
+        } else {
+            // the tile in bucket order: exclusive scan of the counts by warp 0
             if (tid < 32) {
                 uint32_t v[NB / 32];
                 uint32_t run = 0;
@@ -992,51 +1082,28 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) partition_kernel(Part
 #pragma unroll
                 for (int i = 0; i < NB / 32; ++i) sm.loc[tid * (NB / 32) + i] = ex + v[i];
             }
-            if (tid == 0) {
-                // the next tile's keys into the other buffer: its last reader,
-                // the previous tile's write-out, finished before barrier (1)
-                if (a.tma && t_next < ntiles) issue(t_next, b ^ 1);
-                sm.tile_cur = t_next;
-                t_next = claim();
-            }
-            __syncthreads();  // (2) bucket starts within the tile
-
-            // C. stage the keys in bucket order, reusing this tile's buffer
-            K* stage = reinterpret_cast<K*>(sm.buf[b]);
+            if (claimer) next_tile(&sm.tile[turn ^ 1]);
+            __syncthreads();
 #pragma unroll
             for (int r = 0; r < IPT; ++r) {
-                const uint32_t idx = (uint32_t)(r * THREADS + tid);
-                if (FULL || idx < cnt) {
-                    const uint32_t p =
-                        *reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(sm.loc) + (br[r] & 0x7FCu)) +
-                        (br[r] >> 11);
-                    stage[p] = key[r];
-                    sm.bkt[p] = (uint8_t)(br[r] >> 2);
+                const uint32_t b = (br[r] & 0x7FFu) >> 2;
+                if (b < (uint32_t)NB) {
+                    const uint32_t p = sm.loc[b] + (br[r] >> 11);
+                    sm.u.c.stage[p] = key[r];
+                    sm.u.c.bkt[p] = (uint8_t)b;
                 }
             }
             if (tid < NB) {
-                const unsigned long long end = off + h;
-                const bool ovf = !data_ok || end > sm.region_cap[tid];
-                if (ovf && h) raise_error(&a.ctl->err, data_ok ? DEV_ERR_OVERFLOW : DEV_ERR_TIMEOUT);
-                sm.gptr[tid] = reinterpret_cast<uint64_t>(
-                    a.out + (ovf ? a.junk : sm.sd.out_base + sm.region_off[tid] + off) - sm.loc[tid]);
-                sm.hist[tid] = 0;  // (next used after barrier (3))
+                sm.w.ptr[tid] = reinterpret_cast<uint64_t>(
+                    a.out + (overflows() ? a.junk : sm.out_base + sm.region_off[tid] + off) - sm.loc[tid]);
+                sm.hist[tid] = 0;
             }
-            if (tid == 0 && !data_ok) sm.abort = 1;
-            __syncthreads();  // (3) staging complete
-
-            // D. coalesced write-out (an overflowed bucket's keys go to the
-            // overflow area past the regions: the level is redone)
-#pragma unroll
-            for (int r = 0; r < IPT; ++r) {
-                const uint32_t i = (uint32_t)(r * THREADS + tid);
-                if (FULL || i < cnt) reinterpret_cast<K*>(sm.gptr[sm.bkt[i]])[i] = stage[i];
-            }
+            advance();
+            __syncthreads();
+            for (uint32_t i = tid; i < tile_cnt; i += THREADS)
+                reinterpret_cast<K*>(sm.w.ptr[sm.u.c.bkt[i]])[i] = sm.u.c.stage[i];
         }
-        b ^= 1;
     }
-    // after an abort, let a copy still in flight land before the block exits
-    if (a.tma && sm.abort && tid == 0 && sm.tile_cur < ntiles) mbar_wait_bounded(&sm.mbar[b], (phases >> b) & 1u);
 }
 
 // Testing: shrink every bucket capacity of segment 0 (forces an overflow).
