@@ -14,7 +14,6 @@
 #pragma once
 
 #include <cuda_runtime.h>
-#include <cuda/atomic>
 #include <stdint.h>
 
 namespace s512 {
@@ -23,16 +22,11 @@ namespace s512 {
 // status / error word written by kernels (never trap)
 enum : uint32_t {
     DEV_ERR_NONE = 0,
-    DEV_ERR_TIMEOUT = 1u << 0,   // a bounded spin gave up (lookback, queue)
+    DEV_ERR_TIMEOUT = 1u << 0,   // a bounded wait gave up
     DEV_ERR_OVERFLOW = 1u << 1,  // a bucket outgrew its sample-based capacity
     DEV_ERR_BOUNDS = 1u << 2,    // a checked index fell outside its buffer
     DEV_ERR_CAPACITY = 1u << 3,  // a work item is larger than its kernel class
 };
-
-// Iteration cap for every spin on a flag another block writes.  With
-// __nanosleep backoff this is well above any legitimate wait (a predecessor
-// tile takes microseconds) and well below a second.
-constexpr uint32_t SPIN_LIMIT = 1u << 22;
 
 __device__ __forceinline__ void raise_error(uint32_t* err, uint32_t code) {
     if (err) atomicOr(err, code);
@@ -209,19 +203,6 @@ __device__ __forceinline__ T keep_side(T x, T y, bool upper) {
 }
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
-
-// 64-bit device-scope loads / stores of look-back status words.  A status
-// word carries its flag and its count together, and nothing else is read
-// through it, so relaxed atomics suffice; acquire loads would also serialise
-// the look-back window's loads behind one another.
-__device__ __forceinline__ unsigned long long ld_status(const unsigned long long* p) {
-    cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> r(*const_cast<unsigned long long*>(p));
-    return r.load(cuda::memory_order_relaxed);
-}
-__device__ __forceinline__ void st_status(unsigned long long* p, unsigned long long v) {
-    cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> r(*p);
-    r.store(v, cuda::memory_order_relaxed);
-}
 
 // splitmix64 finaliser: counter-based hashing for sample positions
 __device__ __forceinline__ uint64_t mix64(uint64_t z) {

@@ -172,46 +172,32 @@ static int partition_entry(T* data, int* values, size_t left, size_t right, T pi
             S512_CUDA_TRY(cudaMemcpyAsync(dv, values + left, n * sizeof(int), cudaMemcpyHostToDevice, st));
         }
     }
-    constexpr int THREADS = 256, IPT = sizeof(T) == 4 ? 16 : 8;
-    constexpr int TILE = THREADS * IPT;
-    const uint32_t ntiles = (uint32_t)((n + TILE - 1) / TILE);
-    T* ok = (T*)C->get("p2_keys", n * sizeof(T));
-    int* ov = KV ? (int*)C->get("p2_vals", n * sizeof(int)) : nullptr;
-    unsigned long long* status = (unsigned long long*)C->get("p2_status", (size_t)ntiles * 2 * 8 + 16);
+    const Part2Shape sh = part2_shape(n, (uint32_t)C->sms * 8);
+    T* tk = (T*)C->get("p2_keys", n * sizeof(T));
+    int* tv = KV ? (int*)C->get("p2_vals", n * sizeof(int)) : nullptr;
+    unsigned long long* counts = (unsigned long long*)C->get("p2_counts", part2_count_words(sh.blocks) * 8);
     Part2Ctl* ctl = (Part2Ctl*)C->get("p2_ctl", sizeof(Part2Ctl));
     Part2Ctl* hctl = (Part2Ctl*)C->host_pinned(sizeof(Part2Ctl));
-    if (!ok || (KV && !ov) || !status || !ctl || !hctl) return S512_ERR_ALLOC;
-    // (the spare pair of status words past the last tile is the never-written
-    // predecessor of the failure-injection test)
-    S512_CUDA_TRY(cudaMemsetAsync(status, 0, (size_t)(ntiles + 1) * 2 * 8, st));
-    S512_CUDA_TRY(cudaMemsetAsync(ctl, 0, sizeof(Part2Ctl), st));
-    auto fn = partition2_kernel<T, KV, THREADS, IPT>;
-    int grid = 0;
-    S512_CUDA_TRY(launch_persistent(*C, fn, THREADS, 0, st, (int)ntiles, &grid));
-    fn<<<grid, THREADS, 0, st>>>(dk, dv, ok, ov, (uint64_t)n, pivot, status, ctl, ntiles,
-                                 (config().fault_inject & S512_FAULT_TIMEOUT) ? ntiles : 0xFFFFFFFFu);
-    S512_LAUNCH_CHECK();
-    // the error word first: tiles that gave up wrote nothing, so on an error
-    // the scratch holds stale keys and the caller's range stays as it was
+    if (!tk || (KV && !tv) || !counts || !ctl || !hctl) return S512_ERR_ALLOC;
+    S512_CUDA_TRY((launch_part2<T, KV>(dk, dv, tk, tv, (uint64_t)n, pivot, sh, counts, ctl,
+                                       (config().fault_inject & S512_FAULT_TIMEOUT) ? 1 : 0, st)));
     S512_CUDA_TRY(cudaMemcpyAsync(hctl, ctl, sizeof(Part2Ctl), cudaMemcpyDeviceToHost, st));
-    S512_CUDA_TRY(cudaStreamSynchronize(st));
-    if (hctl->err) {
-        guard_.finish();
-        set_error("partition look-back wait timed out");
-        return S512_ERR_TIMEOUT;
-    }
-    T* dst = host ? dk : data + left;
-    S512_CUDA_TRY(cudaMemcpyAsync(dst, ok, n * sizeof(T), cudaMemcpyDeviceToDevice, st));
-    if (KV) S512_CUDA_TRY(cudaMemcpyAsync(host ? dv : values + left, ov, n * sizeof(int), cudaMemcpyDeviceToDevice, st));
     if (host) {
-        S512_CUDA_TRY(cudaMemcpyAsync(data + left, dk, n * sizeof(T), cudaMemcpyDeviceToHost, st));
-        if (KV) S512_CUDA_TRY(cudaMemcpyAsync(values + left, dv, n * sizeof(int), cudaMemcpyDeviceToHost, st));
+        S512_CUDA_TRY(cudaStreamSynchronize(st));
+        if (!hctl->err) {
+            S512_CUDA_TRY(cudaMemcpyAsync(data + left, dk, n * sizeof(T), cudaMemcpyDeviceToHost, st));
+            if (KV) S512_CUDA_TRY(cudaMemcpyAsync(values + left, dv, n * sizeof(int), cudaMemcpyDeviceToHost, st));
+        }
     }
     guard_.finish();
     S512_CUDA_TRY(cudaStreamSynchronize(st));
     s512_stats& S = thread_stats();
     memset(&S, 0, sizeof(S));
-    S.kernel_launches = 1;
+    if (hctl->err) {
+        set_error("partition wait timed out");
+        return S512_ERR_TIMEOUT;
+    }
+    S.kernel_launches = 2;
     S.key_bytes = sizeof(T);
     *boundary = left + (size_t)hctl->total_low;
     return S512_OK;
