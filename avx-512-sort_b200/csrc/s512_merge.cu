@@ -1,6 +1,7 @@
 // s512_merge.cu -- C-ABI entry points for merging sorted runs on the GPU and
 // for the merge-based drivers (SortOmpMerge, SortOmpMergeDeps,
 // SortOmpParMerge: sort512.hpp:6006-6174 with parallelInplace.hpp).
+#include <algorithm>
 #include <vector>
 
 #include "s512_merge.cuh"
@@ -38,19 +39,28 @@ static int merge_tree(DevCtx& C, T* data, T* tmp, std::vector<Run> runs, cudaStr
             pairs.push_back(p);
             next.push_back({p.out0, p.la + p.lb});
         }
-        MergePair* dpairs = (MergePair*)C.get("merge_pairs", pairs.size() * sizeof(MergePair));
+        MergePairs level;
+        level.n = (uint32_t)pairs.size();
+        level.more = nullptr;
+        if (pairs.size() <= MERGE_INLINE) {
+            std::copy(pairs.begin(), pairs.end(), level.p);
+        } else {
+            MergePair* dpairs = (MergePair*)C.get("merge_pairs", pairs.size() * sizeof(MergePair));
+            if (!dpairs) return S512_ERR_ALLOC;
+            S512_CUDA_TRY(cudaMemcpyAsync(dpairs, pairs.data(), pairs.size() * sizeof(MergePair),
+                                          cudaMemcpyHostToDevice, st));
+            // the host vector is reused next level: the copy must have read it
+            S512_CUDA_TRY(cudaStreamSynchronize(st));
+            level.more = dpairs;
+        }
         uint64_t* cor = (uint64_t*)C.get("merge_corank", (size_t)tiles * sizeof(uint64_t));
-        if (!dpairs || !cor) return S512_ERR_ALLOC;
-        S512_CUDA_TRY(cudaMemcpyAsync(dpairs, pairs.data(), pairs.size() * sizeof(MergePair),
-                                      cudaMemcpyHostToDevice, st));
-        corank_kernel<T><<<(tiles + 255) / 256, 256, 0, st>>>(src, dpairs, (uint32_t)pairs.size(), tiles, cor);
+        if (!cor) return S512_ERR_ALLOC;
+        corank_kernel<T><<<(tiles + 256 / CR_LANES - 1) / (256 / CR_LANES), 256, 0, st>>>(src, level, tiles, cor);
         S512_LAUNCH_CHECK();
         int grid = 0;
         S512_CUDA_TRY(launch_persistent(C, merge_kernel<T>, MERGE_THREADS, 0, st, (int)tiles, &grid));
-        merge_kernel<T><<<grid, MERGE_THREADS, 0, st>>>(src, dst, dpairs, (uint32_t)pairs.size(), tiles, cor);
+        merge_kernel<T><<<grid, MERGE_THREADS, 0, st>>>(src, dst, level, tiles, cor);
         S512_LAUNCH_CHECK();
-        // the host vector is reused next level: the copy above must have read it
-        S512_CUDA_TRY(cudaStreamSynchronize(st));
         *launches += 2;
         std::swap(src, dst);
         runs.swap(next);
