@@ -148,7 +148,15 @@ struct Level {
     uint32_t ntiles_bound;
     K* out;
     uint64_t junk;              // offset in out of JUNK_KEYS keys past every region (overflow writes)
+    uint64_t keys;              // keys of the level
+    bool whole;                 // one segment covering an array: `first` is written to segs
+    SegDesc first;
 };
+
+// Levels of up to this many keys queue their leaves before the host has seen
+// the counts (leaf_any_kernel); larger ones read them back and launch each
+// class in blocks of its size.  At 2^22 doubles the two are level.
+constexpr uint64_t BLIND_KEYS = 1u << 22;
 
 template <typename K, typename InCodec, typename UserOut, typename Shape = PartShape<K>>
 static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, size_t n, cudaStream_t st,
@@ -176,8 +184,8 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
     if (!samples || !splits || !counts || (fit && !lsets)) return S512_ERR_ALLOC;
 
     const int t0 = tm.mark();
-    S512_CUDA_TRY(cudaMemsetAsync(ctl, 0, sizeof(LevelCtl), st));
-    S512_CUDA_TRY(cudaMemsetAsync(counts, 0, (size_t)nsegs * NB * sizeof(uint64_t), st));
+    init_level_kernel<<<nsegs, NB, 0, st>>>(ctl, counts, L.whole ? L.segs : nullptr, L.first);
+    S512_LAUNCH_CHECK();
     const uint64_t seed = config().seed + 0x9E3779B97F4A7C15ull * (uint64_t)(level + 1);
     {
         // enough blocks per segment to fill the chip (a fed level reads the
@@ -192,7 +200,7 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
         fn<<<nsegs, SAMPLE_THREADS, split_smem<K>(), st>>>(samples, L.segs, splits, KB, fit ? 1 : 0);
         S512_LAUNCH_CHECK();
     }
-    S.kernel_launches += 2;
+    S.kernel_launches += 3;
     int tfit0 = -1;
     if (fit) {
         // the model is fitted to the same sorted sample; the split set above
@@ -273,9 +281,25 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
     pl.key_bytes = KB;
     plan_kernel<K><<<nsegs, NB, 0, st>>>(pl, nsegs);
     S512_LAUNCH_CHECK();
+    S.kernel_launches += 1;
+    const bool blind = L.keys <= BLIND_KEYS;
+    LeafItem<K>* any_uneven = nullptr;
+    if (blind) {
+        any_uneven = (LeafItem<K>*)C.get("any_uneven", (size_t)nsegs * NB * sizeof(LeafItem<K>));
+        if (!any_uneven) return S512_ERR_ALLOC;
+        auto fn = leaf_any_kernel<K, UserOut>;
+        const size_t smem = SlotSmem<K, ANY_THREADS, 16, false>::bytes;
+        int grid = 0;
+        // (a bucket per block at most, as far as the host can tell)
+        S512_CUDA_TRY(launch_persistent(C, fn, ANY_THREADS, smem, st, (int)std::min<uint64_t>(nsegs * (uint64_t)NB, 1u << 20),
+                                        &grid));
+        fn<<<grid, ANY_THREADS, smem, st>>>(LeafLists<K>{items[0], item_cap}, ctl, uout, any_uneven);
+        S512_LAUNCH_CHECK();
+        S.kernel_launches += 1;
+    }
     S512_CUDA_TRY(cudaMemcpyAsync(host_ctl, ctl, sizeof(LevelCtl), cudaMemcpyDeviceToHost, st));
     S512_CUDA_TRY(cudaStreamSynchronize(st));
-    S.kernel_launches += 1;
+    bool leaves_done = blind && !host_ctl->err;
 
     if (host_ctl->err & DEV_ERR_TIMEOUT) {
         set_error("partition wait timed out at level %d", level);
@@ -288,8 +312,10 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
         if (lsets) S.learned_rejected += host_ctl->learned_used;
         pa.learned = nullptr;
         pl.learned = nullptr;
-        const uint32_t ntiles = L.ntiles_dev ? host_ctl->ntiles_next : L.ntiles_host;
-        (void)ntiles;
+        if (L.tile_seg && nsegs <= (uint32_t)SEG_SMEM) {  // (the pass itself did without the map)
+            tile_map_kernel<<<nsegs, 256, 0, st>>>(L.segs, nsegs, const_cast<uint32_t*>(L.tile_seg));
+            S512_LAUNCH_CHECK();
+        }
         S512_CUDA_TRY(cudaMemsetAsync(counts, 0, (size_t)nsegs * NB * sizeof(uint64_t), st));
         // same tile shape as the partition kernel: tiles are numbered for it
         auto cfn = count_kernel<K, InCodec, Shape::THREADS, Shape::IPT>;
@@ -320,6 +346,21 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
 
     // leaves of this level
     const int t3 = tm.mark();
+    if (leaves_done) {
+        // the largest class's buckets are left, and the uneven ones
+        for (int c = 0; c < ANY_CLASSES; ++c) host_ctl->n_items[c] = 0;
+        host_ctl->n_items[CLS_COPY] = 0;
+        const uint32_t nu = host_ctl->n_uneven[ANY_CLASSES - 1];
+        if (nu) {
+            auto fn = leaf_merge_kernel<K, UserOut, ANY_THREADS, 16>;
+            const size_t smem = (size_t)padded_len(ANY_CAP) * sizeof(K);
+            int grid = 0;
+            S512_CUDA_TRY(launch_persistent(C, fn, ANY_THREADS, smem, st, (int)nu, &grid));
+            fn<<<grid, ANY_THREADS, smem, st>>>(any_uneven, &ctl->n_uneven[ANY_CLASSES - 1], uout);
+            S512_LAUNCH_CHECK();
+            S.kernel_launches += 1;
+        }
+    }
     size_t n_block_items = 0;
     for (int c = 1; c < NCLASS; ++c) n_block_items += host_ctl->n_items[c];
     LeafItem<K>* uneven =
@@ -372,8 +413,8 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
 // several segments are laid out by prepare_level_kernel.  Buckets that fit a
 // leaf are sorted straight into their final place in the caller's array.
 //
-// `whole` says that segs0 is one segment covering the caller's array from
-// element 0 with its tile fields set (sort_pipeline); any other list, even of
+// `whole` says that segs0 is room for one segment covering the caller's array
+// from element 0 (sort_pipeline; the level writes it); any other list, even of
 // one segment, is laid out on the device.
 template <typename K, typename UserIn, typename UserOut>
 static int run_levels(DevCtx& C, UserIn uin, UserOut uout, SegDesc* segs0, uint32_t nsegs0, uint64_t keys0,
@@ -410,6 +451,9 @@ static int run_levels(DevCtx& C, UserIn uin, UserOut uout, SegDesc* segs0, uint3
     L0.nsegs = nsegs0;
     L0.out = T[0];
     L0.junk = need0;
+    L0.keys = keys0;
+    L0.whole = single;
+    L0.first = SegDesc{0, keys0, 0, 0, 0, (uint32_t)((keys0 + TILE_ONE - 1) / TILE_ONE)};
     if (single) {
         L0.tile_seg = nullptr;
         L0.ntiles_host = (uint32_t)((keys0 + TILE_ONE - 1) / TILE_ONE);
@@ -419,12 +463,14 @@ static int run_levels(DevCtx& C, UserIn uin, UserOut uout, SegDesc* segs0, uint3
         const uint32_t bound = (uint32_t)(keys0 / TILE) + nsegs0 + 1;
         uint32_t* tile_seg = (uint32_t*)C.get("tile_seg", (size_t)bound * sizeof(uint32_t));
         if (!tile_seg) return S512_ERR_ALLOC;
-        S512_CUDA_TRY(cudaMemsetAsync(&ctls[1], 0, sizeof(LevelCtl), st));
         prepare_level_kernel<<<1, 1024, 0, st>>>(segs0, nsegs0, TILE, &ctls[1]);
         S512_LAUNCH_CHECK();
-        tile_map_kernel<<<nsegs0, 256, 0, st>>>(segs0, nsegs0, tile_seg);
-        S512_LAUNCH_CHECK();
-        S.kernel_launches += 2;
+        S.kernel_launches += 1;
+        if (nsegs0 > (uint32_t)SEG_SMEM) {
+            tile_map_kernel<<<nsegs0, 256, 0, st>>>(segs0, nsegs0, tile_seg);
+            S512_LAUNCH_CHECK();
+            S.kernel_launches += 1;
+        }
         L0.tile_seg = tile_seg;
         L0.ntiles_host = 0;
         L0.ntiles_dev = &ctls[1].ntiles_next;
@@ -461,12 +507,14 @@ static int run_levels(DevCtx& C, UserIn uin, UserOut uout, SegDesc* segs0, uint3
         if (!tile_seg) return S512_ERR_ALLOC;
         LevelCtl* lctl = &ctls[level & 1];
         LevelCtl* tctl = &ctls[(level + 1) & 1];  // receives this level's tile count
-        S512_CUDA_TRY(cudaMemsetAsync(tctl, 0, sizeof(LevelCtl), st));
         prepare_level_kernel<<<1, 1024, 0, st>>>(cur, nsegs, TILE, tctl);
         S512_LAUNCH_CHECK();
-        tile_map_kernel<<<nsegs, 256, 0, st>>>(cur, nsegs, tile_seg);
-        S512_LAUNCH_CHECK();
-        S.kernel_launches += 2;
+        S.kernel_launches += 1;
+        if (nsegs > (uint32_t)SEG_SMEM) {
+            tile_map_kernel<<<nsegs, 256, 0, st>>>(cur, nsegs, tile_seg);
+            S512_LAUNCH_CHECK();
+            S.kernel_launches += 1;
+        }
         Level<K, Raw<K>> Ln;
         Ln.in = Raw<K>{in_buf, nullptr};
         Ln.segs = cur;
@@ -477,6 +525,9 @@ static int run_levels(DevCtx& C, UserIn uin, UserOut uout, SegDesc* segs0, uint3
         Ln.ntiles_bound = ntiles_bound;
         Ln.out = out_buf;
         Ln.junk = need;
+        Ln.keys = next_keys;
+        Ln.whole = false;
+        Ln.first = SegDesc{};
         // the tile count lives in tctl, so the level's own control block is the other one
         rc = run_level<K, Raw<K>, UserOut>(C, Ln, level, uout, keys0, st, lctl, tctl, nxt, next_cap, tm, S,
                                            host_ctl, learned, host_ctl->max_bucket);
@@ -494,20 +545,11 @@ static int run_levels(DevCtx& C, UserIn uin, UserOut uout, SegDesc* segs0, uint3
 template <typename K, typename UserIn, typename UserOut>
 static int sort_pipeline(DevCtx& C, UserIn uin, UserOut uout, size_t n, cudaStream_t st, bool learned,
                          const HostFeed* feed = nullptr) {
-    constexpr int TILE = PartShapeOne<K>::THREADS * PartShapeOne<K>::IPT;  // a single segment
     s512_stats& S = thread_stats();
     PhaseTimer tm(st, config().collect_stats != 0);
     const int tstart = tm.mark();
     SegDesc* seg0 = (SegDesc*)C.get("seg_whole", sizeof(SegDesc));
     if (!seg0) return S512_ERR_ALLOC;
-    SegDesc s0;
-    s0.in_off = 0;
-    s0.count = n;
-    s0.final_off = 0;
-    s0.out_base = 0;
-    s0.tile_start = 0;
-    s0.ntiles = (uint32_t)((n + TILE - 1) / TILE);
-    S512_CUDA_TRY(cudaMemcpyAsync(seg0, &s0, sizeof(SegDesc), cudaMemcpyHostToDevice, st));
     int rc = run_levels<K, UserIn, UserOut>(C, uin, uout, seg0, 1, n, st, tm, S, true, learned, feed);
     if (rc) return rc;
     const int tend = tm.mark();

@@ -508,6 +508,18 @@ __device__ bool make_direct(const K (&key)[IPT], uint32_t m, uint64_t count, int
     return true;
 }
 
+// Start of a level (one block per segment): its control block and fill
+// counters zeroed and, for a level that is one whole array, its segment
+// written (one launch instead of a copy and two fills).
+static __global__ void __launch_bounds__(NB) init_level_kernel(LevelCtl* ctl, uint64_t* counts, SegDesc* seg,
+                                                               SegDesc whole) {
+    counts[(size_t)blockIdx.x * NB + threadIdx.x] = 0;
+    if (blockIdx.x == 0) {
+        for (uint32_t i = threadIdx.x; i < sizeof(LevelCtl) / 4; i += NB) reinterpret_cast<uint32_t*>(ctl)[i] = 0;
+        if (seg && threadIdx.x == 0) *seg = whole;
+    }
+}
+
 // Keys sampled from every segment, `parts` blocks per segment: random reads
 // are bound by how many one SM can have outstanding, so they are spread over
 // the chip (16384 reads by one block take 13 us to 33 us, by 64 blocks 2.2 us).
@@ -1199,6 +1211,9 @@ __global__ void __launch_bounds__(NB) plan_kernel(PlanArgs<K> a, uint32_t nsegs)
     __shared__ uint64_t wtot64[8];
     const uint32_t s = blockIdx.x;
     if (s >= nsegs) return;
+    // (a pass that reported an error leaves no work: leaves may already be
+    // queued behind this launch)
+    if (a.ctl->err & (DEV_ERR_OVERFLOW | DEV_ERR_TIMEOUT)) return;
     const SegDesc sd = a.segs[s];
     const bool use_learned = a.learned && a.learned[s].ok;
     const uint32_t nbk = use_learned ? a.learned[s].nbuckets : a.splits[s].nbuckets;
@@ -1438,6 +1453,63 @@ __global__ void __launch_bounds__(THREADS, leaf_min_blocks(THREADS))
             key, cur.count, [&](uint32_t i, K x) { out.store(dst + i, x); }, [&]() { load(next); },
             [&]() { uneven[atomicAdd(n_uneven, 1u)] = cur; }, smem_raw, red);
         cur = next;
+    }
+}
+
+// Every bucket of up to ANY_CAP keys of a level, and its copies, in one launch
+// that reads the counts on the device: it is queued behind the plan before the
+// host has seen them, and one size of block sorts all classes.  For levels of
+// few keys, where a read-back and a launch per class cost more than blocks
+// that fit their buckets save (2^20 int32: eight leaf launches and their gaps
+// 45 us, this one MEAS_L us).  The host launches what it leaves: larger
+// buckets, and those found uneven.
+constexpr int ANY_THREADS = 512;
+constexpr int ANY_CLASSES = 8;  // leaf classes 0..7
+constexpr int ANY_CAP = class_cap(ANY_CLASSES - 1);
+static_assert(ANY_CAP == ANY_THREADS * 16, "the largest class fills a block's 16 keys per thread");
+template <typename K>
+struct LeafLists {
+    const LeafItem<K>* items;  // NCLASS + 1 lists of `cap` items each
+    uint32_t cap;
+};
+template <typename K, typename OutCodec>
+__global__ void __launch_bounds__(ANY_THREADS, 2) leaf_any_kernel(LeafLists<K> lists, LevelCtl* ctl, OutCodec out,
+                                                                  LeafItem<K>* uneven) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ SlotRed<K> red;
+    if (ctl->err) return;
+    uint32_t total = ctl->n_items[CLS_COPY];
+#pragma unroll
+    for (int c = 0; c < ANY_CLASSES; ++c) total += ctl->n_items[c];
+    for (uint32_t it = blockIdx.x; it < total; it += gridDim.x) {
+        uint32_t i = it;
+        int c = ANY_CLASSES - 1;  // the largest first, the copies last
+        for (; c >= 0; --c) {
+            const uint32_t n = ctl->n_items[c];
+            if (i < n) break;
+            i -= n;
+        }
+        const LeafItem<K> item = lists.items[(size_t)(c < 0 ? CLS_COPY : c) * lists.cap + i];
+        auto store = [&](uint32_t k, K x) { out.store(item.dst + k, x); };
+        auto give = [&]() { uneven[atomicAdd(&ctl->n_uneven[ANY_CLASSES - 1], 1u)] = item; };
+        auto sort = [&](auto ept) {
+            constexpr int EPT = decltype(ept)::value;
+            K key[EPT];
+#pragma unroll
+            for (int r = 0; r < EPT; ++r) {
+                const uint32_t k = (uint32_t)r * ANY_THREADS + threadIdx.x;
+                if (k < item.count) key[r] = __ldg(item.src + k);
+            }
+            block_slot_sort<K, ANY_THREADS, EPT, false>(key, item.count, store, [] {}, give, smem_raw, red);
+        };
+        if (c < 0) {
+            for (uint32_t k = threadIdx.x; k < item.count; k += ANY_THREADS) store(k, item.src[k]);
+        } else if (item.count > ANY_THREADS * 8) {
+            sort(std::integral_constant<int, 16>{});
+        } else {
+            sort(std::integral_constant<int, 8>{});
+        }
+        __syncthreads();  // (the two sizes lay out shared memory differently)
     }
 }
 
