@@ -67,6 +67,7 @@ __device__ __forceinline__ uint64_t enc_kv(int key, int val) {
 template <typename K>
 struct Raw {
     using Key = K;
+    static constexpr bool PAIRS = false;  // words of key and value
     const K* __restrict__ in;
     K* __restrict__ out;
     __device__ __forceinline__ K raw(size_t i) const { return __ldg(in + i); }
@@ -79,6 +80,7 @@ struct Raw {
 
 struct CodecI32 {
     using Key = uint32_t;
+    static constexpr bool PAIRS = false;
     const int* __restrict__ in;
     int* __restrict__ out;
     __device__ __forceinline__ uint32_t raw(size_t i) const { return (uint32_t)__ldg(in + i); }
@@ -90,6 +92,7 @@ struct CodecI32 {
 
 struct CodecF64 {
     using Key = uint64_t;
+    static constexpr bool PAIRS = false;
     const unsigned long long* __restrict__ in;
     unsigned long long* __restrict__ out;
     __device__ __forceinline__ uint64_t raw(size_t i) const { return __ldg(in + i); }
@@ -103,6 +106,7 @@ struct CodecF64 {
 
 struct CodecKV {
     using Key = uint64_t;
+    static constexpr bool PAIRS = true;
     const int* __restrict__ kin;
     const int* __restrict__ vin;
     int* __restrict__ kout;
@@ -124,6 +128,7 @@ struct CodecKV {
 // int64 keys: uint64 k = x ^ 2^63 (signed order).
 struct CodecI64 {
     using Key = uint64_t;
+    static constexpr bool PAIRS = false;
     const unsigned long long* __restrict__ in;
     unsigned long long* __restrict__ out;
     __device__ __forceinline__ uint64_t raw(size_t i) const { return __ldg(in + i); }
@@ -139,6 +144,7 @@ struct CodecI64 {
 // word per pair (little-endian: key in the low half), encoded like CodecKV.
 struct CodecKVPairs {
     using Key = uint64_t;
+    static constexpr bool PAIRS = true;
     const unsigned long long* __restrict__ in;
     unsigned long long* __restrict__ out;
     __device__ __forceinline__ uint64_t raw(size_t i) const { return __ldg(in + i); }

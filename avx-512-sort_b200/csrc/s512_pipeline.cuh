@@ -23,8 +23,7 @@ template <> struct PartShapeOne<uint64_t> { static constexpr int THREADS = 512, 
 // ---------------------------------------------------------------------------
 // leaf launches per class
 
-// Slot sort of a class's buckets, then the block sort of those it found
-// uneven (the second launch reads the count on the device and exits at once
+// Slot sort of a class's buckets, then those it found uneven (the second launch reads the count on the device and exits at once
 // when there are none).
 template <typename K, typename OutCodec, int THREADS, int EPT>
 static int launch_leaf_block(DevCtx& C, const LeafItem<K>* items, uint32_t n, OutCodec out, LeafItem<K>* uneven,
@@ -38,8 +37,8 @@ static int launch_leaf_block(DevCtx& C, const LeafItem<K>* items, uint32_t n, Ou
         S512_LAUNCH_CHECK();
     }
     {
-        auto fn = leaf_merge_kernel<K, OutCodec, THREADS, EPT>;
-        const size_t smem = (size_t)padded_len(THREADS * EPT) * sizeof(K);
+        auto fn = leaf_uneven_kernel<K, OutCodec, THREADS, EPT>;
+        const size_t smem = leaf_uneven_smem<K, OutCodec, THREADS, EPT>();
         int grid = 0;
         S512_CUDA_TRY(launch_persistent(C, fn, THREADS, smem, st, (int)n, &grid));
         fn<<<grid, THREADS, smem, st>>>(uneven, n_uneven, out);
@@ -197,7 +196,8 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
         S512_LAUNCH_CHECK();
         auto fn = split_kernel<K>;
         S512_CUDA_TRY(C.prepare((const void*)fn, split_smem<K>()));
-        fn<<<nsegs, SAMPLE_THREADS, split_smem<K>(), st>>>(samples, L.segs, splits, KB, fit ? 1 : 0);
+        fn<<<nsegs, SAMPLE_THREADS, split_smem<K>(), st>>>(samples, L.segs, splits, KB, fit ? 1 : 0,
+                                                              UserOut::PAIRS ? 1 : 0);
         S512_LAUNCH_CHECK();
     }
     S.kernel_launches += 3;
@@ -352,8 +352,8 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
         host_ctl->n_items[CLS_COPY] = 0;
         const uint32_t nu = host_ctl->n_uneven[ANY_CLASSES - 1];
         if (nu) {
-            auto fn = leaf_merge_kernel<K, UserOut, ANY_THREADS, 16>;
-            const size_t smem = (size_t)padded_len(ANY_CAP) * sizeof(K);
+            auto fn = leaf_uneven_kernel<K, UserOut, ANY_THREADS, 16>;
+            const size_t smem = leaf_uneven_smem<K, UserOut, ANY_THREADS, 16>();
             int grid = 0;
             S512_CUDA_TRY(launch_persistent(C, fn, ANY_THREADS, smem, st, (int)nu, &grid));
             fn<<<grid, ANY_THREADS, smem, st>>>(any_uneven, &ctl->n_uneven[ANY_CLASSES - 1], uout);

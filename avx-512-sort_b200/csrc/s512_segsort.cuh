@@ -147,9 +147,9 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
         next.count = 0;
         if (nx < nitems) next = items[nx];
         const uint64_t off = cur.off;
-        block_slot_sort<K, THREADS, EPT, true>(
+        block_slot_sort<K, THREADS, EPT, SLOT_INLINE>(
             key, cur.count, [&](uint32_t i, K x) { io.store(off + i, x); }, [&]() { load(next); }, [] {}, smem_raw,
-            red);
+            red, !Codec::PAIRS);
         cur = next;
     }
 }

@@ -12,9 +12,10 @@
 // per key, where a comparison network costs one compare-exchange per key for
 // every stage.  When the spread is uneven (a cluster, a run of repeated
 // values, an outlier that stretches the range) the slot counts show it before
-// any key moves: if a slot holds more than SLOT_MAX keys, or some thread's
-// keys met more than SLOT_MEET others each on average, the bucket is sorted
-// by the bitonic + merge-path block sort instead (s512_blocksort.cuh).
+// any key moves: if a slot holds SLOT_MAX keys or more, or some thread's
+// keys met more than SLOT_MEET others each on average, the bucket is dealt
+// again through slots refined by the first counts (refine_slots), and by the
+// bitonic + merge-path block sort (s512_blocksort.cuh) if those are uneven too.
 //
 // What bounds it: issue slots and shared-memory latency, not HBM, so the code
 // is laid out for few instructions per key.  Four 8-bit slot counters share a
@@ -102,16 +103,19 @@ struct SlotRed {
 };
 
 // Shared memory of block_slot_sort for a block of THREADS x IPT keys: the
-// key buffer (padded for the block sort when that runs inline, INLINE), one
-// word of four slot counters per key, and the list of the slots that received
-// several keys (at most half as many as keys).
+// key buffer, one word of four slot counters per key, and the list of the
+// slots that received several keys (at most half as many as keys; before that
+// list is written its space holds the big slots of refine_slots).  The block
+// sort, where it may run (INLINE), lays its padded keys over all of it.
 template <typename K, int THREADS, int IPT, bool INLINE = true>
 struct SlotSmem {
     static constexpr uint32_t S = (uint32_t)THREADS * IPT;
-    static constexpr size_t keys_bytes = ((size_t)(INLINE ? padded_len(S) : S) * sizeof(K) + 15) & ~(size_t)15;
+    static constexpr size_t keys_bytes = (size_t)S * sizeof(K);
     static constexpr size_t ctr_bytes = (size_t)S * sizeof(uint32_t);
     static constexpr size_t list_bytes = (size_t)S;
-    static constexpr size_t bytes = keys_bytes + ctr_bytes + list_bytes;
+    static constexpr size_t slot_bytes = keys_bytes + ctr_bytes + list_bytes;
+    static constexpr size_t padded_bytes = ((size_t)padded_len(S) * sizeof(K) + 15) & ~(size_t)15;
+    static constexpr size_t bytes = INLINE && padded_bytes > slot_bytes ? padded_bytes : slot_bytes;
 };
 
 // Byte offset of a counter word in shared memory.  A thread scans IPT
@@ -190,6 +194,152 @@ __device__ __forceinline__ void block_bounds(const K (&key)[IPT], uint32_t c, Sl
     }
 }
 
+enum SlotMode { SLOT_HAND, SLOT_INLINE, SLOT_REFINE };
+
+// A coarse slot of more than SLOT_MAX keys: its keys' own bounds, as a map to
+// four fine slots per key.
+template <typename K>
+struct alignas(16) BigSlot {
+    K lo;
+    uint32_t mul;   // (the slot's count until its bounds are known)
+    uint32_t aux;   // first place | shift << 16 | direct << 22 | all equal << 23
+};
+
+// Fine slots for a bucket whose values crowd: every key's slot of 4*c, rising
+// with the keys, into fine[].  The bucket is dealt once into as many coarse
+// slots as the class has keys; the keys of a coarse slot then spread over four
+// fine slots per key, by their place between the slot's own lowest and highest
+// key where it holds many (a cluster, a hot key's values: exact bounds, found
+// by a warp from the dealt keys; equal keys by their rank, so that any number
+// of them fits), by their place in the slot where it holds few.
+// Leaves the counters zeroed, a barrier behind.
+template <typename K, int THREADS, int IPT>
+__device__ __forceinline__ void refine_slots(const K (&key)[IPT], uint32_t c, K lo, K range, uint32_t (&fine)[IPT],
+                                             K* s, unsigned char* ctr, BigSlot<K>* big, SlotRed<K>& red) {
+    constexpr uint32_t S = (uint32_t)THREADS * IPT;
+    constexpr int NW = THREADS / 32;
+    constexpr uint32_t BIG = 0x80000000u;
+    const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    auto zero = [&]() {
+#pragma unroll
+        for (int r = 0; r < IPT; r += 4)
+            *reinterpret_cast<uint4*>(ctr + (size_t)tid * IPT * 4 + r * 4) = make_uint4(0u, 0u, 0u, 0u);
+    };
+    auto quad = [&](int j) {
+        return reinterpret_cast<uint4*>(ctr + ctr_swizzle<IPT>(tid * IPT * 4 + (uint32_t)j * 16));
+    };
+    zero();
+    __syncthreads();
+    // coarse counts; a key's rank in its slot
+    const SlotMap<K> f = make_slot_map_fast<K>(lo, range, S);
+#pragma unroll
+    for (int r = 0; r < IPT; ++r) {
+        if ((uint32_t)r * THREADS + tid < c) {
+            const uint32_t a = ctr_swizzle<IPT>(f(key[r]) * 4u);
+            fine[r] = a | (atomicAdd(reinterpret_cast<uint32_t*>(ctr + a), 1u) << 16);  // (both under 2^16)
+        }
+    }
+    __syncthreads();
+    // places (low half) and numbers of big slots (high half) before each word
+    uint32_t v = 0;
+#pragma unroll
+    for (int j = 0; j < IPT / 4; ++j) {
+        const uint4 q = *quad(j);
+        v += q.x + q.y + q.z + q.w;
+        v += ((q.x > SLOT_MAX ? 1u : 0u) + (q.y > SLOT_MAX ? 1u : 0u) + (q.z > SLOT_MAX ? 1u : 0u) +
+              (q.w > SLOT_MAX ? 1u : 0u)) << 16;
+    }
+    uint32_t inc = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, inc, d);
+        if (lane >= (unsigned)d) inc += o;
+    }
+    if (lane == 31) red.wtot[warp] = inc;
+    __syncthreads();
+    const uint32_t wt = lane < (unsigned)NW ? red.wtot[lane] : 0u;
+    uint32_t run = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? wt : 0u) + inc - v;
+    const uint32_t nbig = __reduce_add_sync(0xFFFFFFFFu, wt) >> 16;  // (at most S / 16)
+#pragma unroll
+    for (int j = 0; j < IPT / 4; ++j) {
+        uint4* qp = quad(j);
+        uint4 q = *qp;
+        auto word = [&](uint32_t n) {  // first place (14 bits), then the count or the big slot's number
+            const uint32_t at = run & 0xFFFFu, id = run >> 16;
+            uint32_t w = (at & 0x3FFFu) | (n << 14);
+            run += n;
+            if (n > SLOT_MAX) {
+                big[id].mul = n;
+                big[id].aux = at;
+                w = BIG | (at & 0x3FFFu) | (id << 14);
+                run += 1u << 16;
+            }
+            return w;
+        };
+        q.x = word(q.x);
+        q.y = word(q.y);
+        q.z = word(q.z);
+        q.w = word(q.w);
+        *qp = q;
+    }
+    __syncthreads();
+    // deal into the coarse slots; keep what a key needs of its slot
+#pragma unroll
+    for (int r = 0; r < IPT; ++r) {
+        if ((uint32_t)r * THREADS + tid < c) {
+            const uint32_t w = *reinterpret_cast<const uint32_t*>(ctr + (fine[r] & 0xFFFFu));
+            const uint32_t rank = fine[r] >> 16;
+            s[(w & 0x3FFFu) + rank] = key[r];
+            fine[r] = (w & BIG) ? (w & ~0x3FFFu) | rank : w;
+        }
+    }
+    __syncthreads();
+    zero();
+    for (uint32_t id = warp; id < nbig; id += NW) {
+        const uint32_t n = big[id].mul, at = big[id].aux;
+        K mn = KeyMax<K>::value, mx = K(0);
+#pragma unroll 4
+        for (uint32_t i = lane; i < n; i += 32) {
+            const K x = s[at + i];
+            mn = kmin(mn, x);
+            mx = kmax(mx, x);
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            mn = kmin(mn, shfl_xor(mn, d));
+            mx = kmax(mx, shfl_xor(mx, d));
+        }
+        const SlotMap<K> g = make_slot_map_fast<K>(mn, mx - mn, 4 * n);
+        __syncwarp();
+        if (lane == 0) {
+            BigSlot<K> b;
+            b.lo = mn;
+            b.mul = g.mul;
+            b.aux = at | (g.sh << 16) | (g.direct << 22) | (mn == mx ? 1u << 23 : 0u);
+            big[id] = b;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < IPT; ++r) {
+        if ((uint32_t)r * THREADS + tid < c) {
+            const uint32_t w = fine[r];
+            uint32_t first, sub;
+            if (w & BIG) {
+                const BigSlot<K> b = big[(w >> 14) & 0x3FFu];
+                first = b.aux & 0xFFFFu;
+                const uint32_t d = (uint32_t)((key[r] - b.lo) >> ((b.aux >> 16) & 63u));
+                sub = (b.aux >> 23) ? 4u * (w & 0x3FFFu) : (b.aux >> 22) ? d : __umulhi(d, b.mul);
+            } else {
+                first = w & 0x3FFFu;
+                const uint32_t d = (uint32_t)((key[r] - lo) >> f.sh);
+                sub = f.direct ? 0u : __umulhi(d * f.mul, 4u * (w >> 14));  // (the fraction of the slot)
+            }
+            fine[r] = 4u * first + sub;
+        }
+    }
+}
+
 // Sort the c <= THREADS*IPT keys held striped in key[] (element
 // r*THREADS + tid in key[r]; entries past c are ignored) into store(0..c).
 // `smem` holds SlotSmem<K,THREADS,IPT>::bytes; `red` is the block's reduction
@@ -201,21 +351,29 @@ __device__ __forceinline__ void block_bounds(const K (&key)[IPT], uint32_t c, Sl
 // barriers), anything else needs a barrier first.
 // Returns how the bucket was sorted, hence where its sorted keys are left in
 // the key buffer: in order (SLOT_EVEN), in the block sort's padded layout
-// (SLOT_UNEVEN, with INLINE_FALLBACK), or nowhere (SLOT_EQUAL).
+// (SLOT_UNEVEN, where the block sort ran), or nowhere (SLOT_EQUAL).
 //
-// An uneven bucket is sorted here by the block sort when INLINE_FALLBACK is
-// set; otherwise thread 0 calls uneven() (which hands the bucket to a
-// separate launch) and nothing is written.  Keeping the block sort out of
-// the kernel keeps the slot path's register budget for the keys.
-template <typename K, int THREADS, int IPT, bool INLINE_FALLBACK, typename Store, typename Refill, typename Uneven>
+// What happens to an uneven bucket depends on MODE.  SLOT_HAND: thread 0 calls
+// uneven() (which hands the bucket to a separate launch) and nothing is
+// written; keeping the rest out of the kernel keeps the slot path's register
+// budget for the keys.  SLOT_INLINE: it is dealt a second time, through slots
+// refined by the first (refine below), and if that leaves it uneven too it is
+// sorted by the block sort.  SLOT_REFINE: the same without the first attempt,
+// for buckets known to be uneven.  `refine` off leaves the second dealing out:
+// words of key/value pairs crowd by hot keys, whose values share their coarse
+// slot with a few other keys that stretch its bounds, so refined slots are
+// rarely even (2^27 pairs with Zipf keys: uneven leaves 1.11 ms by the block
+// sort, 1.54 ms with a second dealing before it).  Doubles gain: a sample of
+// 16384 normal doubles (two signs, 60 binades) is sorted in 45 instead of 72 us.
+template <typename K, int THREADS, int IPT, SlotMode MODE, typename Store, typename Refill, typename Uneven>
 __device__ SlotPath block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refill refill, Uneven uneven,
-                                unsigned char* smem, SlotRed<K>& red) {
+                                unsigned char* smem, SlotRed<K>& red, bool refine = true) {
     constexpr uint32_t S = (uint32_t)THREADS * IPT;
     constexpr uint32_t NSLOTS = 4 * S;
     constexpr int NW = THREADS / 32;
     static_assert(IPT % 4 == 0 && IPT <= 16, "counter words are read four at a time");
     static_assert(S <= 16384, "a place is 14 bits, a counter's byte offset 16");
-    using SM = SlotSmem<K, THREADS, IPT, INLINE_FALLBACK>;
+    using SM = SlotSmem<K, THREADS, IPT, MODE != SLOT_HAND>;
     K* s = reinterpret_cast<K*>(smem);
     unsigned char* ctr = smem + SM::keys_bytes;
     uint16_t* list = reinterpret_cast<uint16_t*>(smem + SM::keys_bytes + SM::ctr_bytes);
@@ -243,25 +401,40 @@ __device__ SlotPath block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refi
     // the key's own increment.  (A byte that passes 255 carries into its
     // neighbour, but then a key has seen the rank SLOT_MAX and the counts are
     // not used.)
-    const SlotMap<K> f = make_slot_map_fast<K>(lo, range, NSLOTS);
     uint32_t pr[IPT];  // counter byte offset | slot within the word | rank << 16
-    uint32_t rmax = 0, rsum = 0, nmulti = 0;
+    uint32_t nmulti = 0;
+    auto count = [&](uint32_t meet, auto slot_of) {
+        uint32_t rmax = 0, rsum = 0;
+        nmulti = 0;
 #pragma unroll
-    for (int r = 0; r < IPT; ++r) {
-        pr[r] = 0;
-        if ((uint32_t)r * THREADS + tid < c) {
-            const uint32_t slot = f(key[r]);
-            const uint32_t a = ctr_swizzle<IPT>(slot & ~3u);
-            const uint32_t k8 = slot << 3;  // (shifts take it modulo 32)
-            const uint32_t old = atomicAdd(reinterpret_cast<uint32_t*>(ctr + a), __funnelshift_l(0u, 1u, k8));
-            const uint32_t rank = __funnelshift_r(old, 0u, k8) & 0xFFu;
-            pr[r] = (a | (slot & 3u)) + (rank << 16);
-            rmax = max(rmax, rank);
-            rsum += rank;
-            nmulti += rank == 1u ? 1u : 0u;
+        for (int r = 0; r < IPT; ++r) {
+            const uint32_t was = MODE == SLOT_HAND ? 0u : pr[r];
+            pr[r] = 0;
+            if ((uint32_t)r * THREADS + tid < c) {
+                const uint32_t slot = slot_of(r, was);
+                const uint32_t a = ctr_swizzle<IPT>(slot & ~3u);
+                const uint32_t k8 = slot << 3;  // (shifts take it modulo 32)
+                const uint32_t old = atomicAdd(reinterpret_cast<uint32_t*>(ctr + a), __funnelshift_l(0u, 1u, k8));
+                const uint32_t rank = __funnelshift_r(old, 0u, k8) & 0xFFu;
+                pr[r] = (a | (slot & 3u)) + (rank << 16);
+                rmax = max(rmax, rank);
+                rsum += rank;
+                nmulti += rank == 1u ? 1u : 0u;
+            }
+        }
+        return !__syncthreads_or(rmax >= SLOT_MAX || rsum > meet * IPT);
+    };
+    bool even = false;
+    if constexpr (MODE != SLOT_REFINE) {
+        const SlotMap<K> f = make_slot_map_fast<K>(lo, range, NSLOTS);
+        even = count(SLOT_MEET, [&](int r, uint32_t) { return f(key[r]); });
+    }
+    if constexpr (MODE != SLOT_HAND) {
+        if (!even && refine) {
+            refine_slots<K, THREADS, IPT>(key, c, lo, range, pr, s, ctr, reinterpret_cast<BigSlot<K>*>(list), red);
+            even = count(2 * SLOT_MEET, [&](int, uint32_t was) { return was; });
         }
     }
-    const bool even = !__syncthreads_or(rmax >= SLOT_MAX || rsum > SLOT_MEET * IPT);
 
     if (even) {
         // 3. exclusive scan of the counts (IPT consecutive words per thread)
@@ -361,7 +534,7 @@ __device__ SlotPath block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refi
         __syncthreads();
         // 6. every key is in its final place
         for (uint32_t p = tid; p < c; p += THREADS) store(p, s[p]);
-    } else if constexpr (INLINE_FALLBACK) {
+    } else if constexpr (MODE != SLOT_HAND) {
         // uneven spread: bitonic leaves + merge path on the same keys
 #pragma unroll
         for (int r = 0; r < IPT; ++r) {

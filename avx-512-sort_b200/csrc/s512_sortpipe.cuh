@@ -551,7 +551,7 @@ constexpr size_t split_smem() { return SlotSmem<K, SAMPLE_THREADS, SAMPLE_IPT>::
 template <typename K>
 __global__ void __launch_bounds__(SAMPLE_THREADS)
     split_kernel(K* __restrict__ samples, const SegDesc* __restrict__ segs, SplitSet<K>* __restrict__ splits,
-                 int key_bytes, int keep_sorted) {
+                 int key_bytes, int keep_sorted, int pairs) {
     using SM = SlotSmem<K, SAMPLE_THREADS, SAMPLE_IPT>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ SlotRed<K> red;
@@ -571,12 +571,12 @@ __global__ void __launch_bounds__(SAMPLE_THREADS)
     const K any = key[0];  // (m >= SAMPLE_THREADS)
     // sorted in registers and shared memory, where the splitters are searched;
     // back to global memory only for the learned fit
-    const SlotPath how = block_slot_sort<K, SAMPLE_THREADS, SAMPLE_IPT, true>(
-        key, m, [&](uint32_t i, K x) { if (keep_sorted) g[i] = x; }, [] {}, [] {}, smem_raw, red);
+    const SlotPath how = block_slot_sort<K, SAMPLE_THREADS, SAMPLE_IPT, SLOT_REFINE>(
+        key, m, [&](uint32_t i, K x) { if (keep_sorted) g[i] = x; }, [] {}, [] {}, smem_raw, red, !pairs);
     __syncthreads();
     const K* sorted = reinterpret_cast<const K*>(smem_raw);
-    static_assert(sizeof(SplitScratch<K>) <= SM::ctr_bytes, "the counters' space is reused");
-    SplitScratch<K>& w = *reinterpret_cast<SplitScratch<K>*>(smem_raw + SM::keys_bytes);
+    static_assert(SM::padded_bytes + sizeof(SplitScratch<K>) <= SM::bytes, "the space behind the keys is reused");
+    SplitScratch<K>& w = *reinterpret_cast<SplitScratch<K>*>(smem_raw + SM::padded_bytes);
     make_splitters<K>(
         [&](uint32_t i) { return how == SLOT_EQUAL ? any : sorted[how == SLOT_EVEN ? i : pidx(i)]; }, m, count, nb,
         splits + s, w);
@@ -1424,7 +1424,7 @@ __host__ __device__ constexpr int leaf_min_blocks(int threads) {
 // into value slots (s512_slotsort.cuh).  The next bucket's keys are loaded
 // into registers while the current one is ranked and written.  A bucket whose
 // slots come out uneven is appended to `uneven` (count in *n_uneven) for
-// leaf_merge_kernel.
+// leaf_uneven_kernel.
 template <typename K, typename OutCodec, int THREADS, int EPT>
 __global__ void __launch_bounds__(THREADS, leaf_min_blocks(THREADS))
     leaf_block_kernel(const LeafItem<K>* __restrict__ items, uint32_t nitems, OutCodec out, LeafItem<K>* uneven,
@@ -1449,7 +1449,7 @@ __global__ void __launch_bounds__(THREADS, leaf_min_blocks(THREADS))
         next.count = 0;
         if (nx < nitems) next = items[nx];
         const size_t dst = cur.dst;
-        block_slot_sort<K, THREADS, EPT, false>(
+        block_slot_sort<K, THREADS, EPT, SLOT_HAND>(
             key, cur.count, [&](uint32_t i, K x) { out.store(dst + i, x); }, [&]() { load(next); },
             [&]() { uneven[atomicAdd(n_uneven, 1u)] = cur; }, smem_raw, red);
         cur = next;
@@ -1500,7 +1500,7 @@ __global__ void __launch_bounds__(ANY_THREADS, 2) leaf_any_kernel(LeafLists<K> l
                 const uint32_t k = (uint32_t)r * ANY_THREADS + threadIdx.x;
                 if (k < item.count) key[r] = __ldg(item.src + k);
             }
-            block_slot_sort<K, ANY_THREADS, EPT, false>(key, item.count, store, [] {}, give, smem_raw, red);
+            block_slot_sort<K, ANY_THREADS, EPT, SLOT_HAND>(key, item.count, store, [] {}, give, smem_raw, red);
         };
         if (c < 0) {
             for (uint32_t k = threadIdx.x; k < item.count; k += ANY_THREADS) store(k, item.src[k]);
@@ -1513,20 +1513,39 @@ __global__ void __launch_bounds__(ANY_THREADS, 2) leaf_any_kernel(LeafLists<K> l
     }
 }
 
-// The buckets leaf_block_kernel found uneven: bitonic leaves + merge path.
+// The buckets the slot sort found uneven.  Of key/value pairs (see
+// block_slot_sort on `refine`): bitonic leaves + merge path; of other keys:
+// refined slots, and that where they are uneven too.
 template <typename K, typename OutCodec, int THREADS, int EPT>
-__global__ void __launch_bounds__(THREADS) leaf_merge_kernel(const LeafItem<K>* __restrict__ items,
-                                                             const uint32_t* n_items, OutCodec out) {
+__global__ void __launch_bounds__(THREADS, OutCodec::PAIRS || 1024 / THREADS < 2 ? 1024 / THREADS : 2)
+    leaf_uneven_kernel(const LeafItem<K>* __restrict__ items, const uint32_t* n_items, OutCodec out) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    K* s = reinterpret_cast<K*>(smem_raw);
     const uint32_t nitems = *n_items;
     for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x) {
         const LeafItem<K> item = items[it];
-        for (uint32_t i = threadIdx.x; i < item.count; i += THREADS) s[pidx(i)] = item.src[i];
-        block_merge_sort<K, THREADS, EPT>(s, item.count);
-        for (uint32_t i = threadIdx.x; i < item.count; i += THREADS) out.store(item.dst + i, s[pidx(i)]);
-        __syncthreads();
+        if constexpr (OutCodec::PAIRS) {
+            K* s = reinterpret_cast<K*>(smem_raw);
+            for (uint32_t i = threadIdx.x; i < item.count; i += THREADS) s[pidx(i)] = item.src[i];
+            block_merge_sort<K, THREADS, EPT>(s, item.count);
+            for (uint32_t i = threadIdx.x; i < item.count; i += THREADS) out.store(item.dst + i, s[pidx(i)]);
+        } else {
+            __shared__ SlotRed<K> red;
+            K key[EPT];
+#pragma unroll
+            for (int r = 0; r < EPT; ++r) {
+                const uint32_t i = (uint32_t)r * THREADS + threadIdx.x;
+                if (i < item.count) key[r] = __ldg(item.src + i);
+            }
+            block_slot_sort<K, THREADS, EPT, SLOT_REFINE>(
+                key, item.count, [&](uint32_t i, K x) { out.store(item.dst + i, x); }, [] {}, [] {}, smem_raw, red);
+        }
+        __syncthreads();  // (the next bucket's keys go where other threads may still read these)
     }
+}
+template <typename K, typename OutCodec, int THREADS, int EPT>
+constexpr size_t leaf_uneven_smem() {
+    using SM = SlotSmem<K, THREADS, EPT>;
+    return OutCodec::PAIRS ? SM::padded_bytes : SM::bytes;
 }
 
 // Copy equality buckets (and single keys) to their final place.
@@ -1572,7 +1591,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) small_block_sort_kern
         const uint32_t i = (uint32_t)r * THREADS + threadIdx.x;
         if (i < n) key[r] = in.load(i);
     }
-    block_slot_sort<K, THREADS, EPT, true>(
-        key, n, [&](uint32_t i, K x) { out.store(i, x); }, [] {}, [] {}, smem_raw, red);
+    block_slot_sort<K, THREADS, EPT, SLOT_INLINE>(
+        key, n, [&](uint32_t i, K x) { out.store(i, x); }, [] {}, [] {}, smem_raw, red, !OutCodec::PAIRS);
 }
 }  // namespace s512
