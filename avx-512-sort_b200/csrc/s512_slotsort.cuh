@@ -12,7 +12,7 @@
 // per key, where a comparison network costs one compare-exchange per key for
 // every stage.  When the spread is uneven (a cluster, a run of repeated
 // values, an outlier that stretches the range) the slot counts show it before
-// any key moves: if a slot holds SLOT_MAX keys or more, or some thread's
+// any key moves: if a slot holds more than SLOT_MAX keys, or some thread's
 // keys met more than SLOT_MEET others each on average, the bucket is dealt
 // again through slots refined by the first counts (refine_slots), and by the
 // bitonic + merge-path block sort (s512_blocksort.cuh) if those are uneven too.
@@ -36,7 +36,7 @@
 
 namespace s512 {
 
-constexpr uint32_t SLOT_MAX = 15;   // largest slot put in order by one thread (4 * 15 < 64: the
+constexpr uint32_t SLOT_MAX = 16;   // largest slot put in order by one thread (3 * 16 < 64: the
                                     // running counts of a word fit their 6 bits)
 constexpr uint32_t SLOT_MEET = 3;   // a thread's keys may meet this many earlier keys each, on average
 
@@ -130,6 +130,13 @@ __device__ __forceinline__ uint32_t ctr_swizzle(uint32_t a) {
     else return a;
 }
 
+// How many of the c keys held striped in key[] this thread holds (key[r] is
+// one for r below that: a compare with a constant per key and phase).
+template <int THREADS>
+__device__ __forceinline__ int own_keys(uint32_t c) {
+    return threadIdx.x < c ? (int)((c - threadIdx.x + THREADS - 1) / THREADS) : 0;
+}
+
 // Bounds of the c keys held striped in key[]: lo <= every key <= lo + range.
 // Of 64-bit keys only the high words are compared: unless they span very few
 // values, the bounds need no more precision (range == 0 is always exact).
@@ -138,10 +145,11 @@ template <typename K, int THREADS, int IPT>
 __device__ __forceinline__ void block_bounds(const K (&key)[IPT], uint32_t c, SlotRed<K>& red, K& lo, K& range) {
     constexpr int NW = THREADS / 32;
     const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    const int own = own_keys<THREADS>(c);
     uint32_t hmin = 0xFFFFFFFFu, hmax = 0u;
 #pragma unroll
     for (int r = 0; r < IPT; ++r) {
-        if ((uint32_t)r * THREADS + tid < c) {
+        if (r < own) {
             const uint32_t h = sizeof(K) == 8 ? (uint32_t)((uint64_t)key[r] >> 32) : (uint32_t)key[r];
             hmin = min(hmin, h);
             hmax = max(hmax, h);
@@ -163,7 +171,7 @@ __device__ __forceinline__ void block_bounds(const K (&key)[IPT], uint32_t c, Sl
             K mn = KeyMax<K>::value, mx = K(0);
 #pragma unroll
             for (int r = 0; r < IPT; ++r) {
-                if ((uint32_t)r * THREADS + tid < c) {
+                if (r < own) {
                     mn = kmin(mn, key[r]);
                     mx = kmax(mx, key[r]);
                 }
@@ -266,7 +274,7 @@ __device__ __forceinline__ void refine_slots(const K (&key)[IPT], uint32_t c, K 
         uint4 q = *qp;
         auto word = [&](uint32_t n) {  // first place (14 bits), then the count or the big slot's number
             const uint32_t at = run & 0xFFFFu, id = run >> 16;
-            uint32_t w = (at & 0x3FFFu) | (n << 14);
+            uint32_t w = (at & 0x3FFFu) | (n << 14);  // (5 bits)
             run += n;
             if (n > SLOT_MAX) {
                 big[id].mul = n;
@@ -385,6 +393,7 @@ __device__ SlotPath block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refi
         *reinterpret_cast<uint4*>(ctr + (size_t)tid * IPT * 4 + r * 4) = make_uint4(0u, 0u, 0u, 0u);
     K lo, range;
     block_bounds<K, THREADS, IPT>(key, c, red, lo, range);
+    const int own = own_keys<THREADS>(c);
 
     if (range == 0) {  // every key equal: already in order
 #pragma unroll
@@ -399,30 +408,31 @@ __device__ SlotPath block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refi
 
     // 2. slot counts: a key's rank in its slot is its counter's byte before
     // the key's own increment.  (A byte that passes 255 carries into its
-    // neighbour, but then a key has seen the rank SLOT_MAX and the counts are
-    // not used.)
+    // neighbour, but then a key has seen a rank of SLOT_MAX or more and the
+    // counts are not used.)
     uint32_t pr[IPT];  // counter byte offset | slot within the word | rank << 16
     uint32_t nmulti = 0;
     auto count = [&](uint32_t meet, auto slot_of) {
-        uint32_t rmax = 0, rsum = 0;
+        uint32_t seen = 0, rsum = 0;
         nmulti = 0;
 #pragma unroll
         for (int r = 0; r < IPT; ++r) {
             const uint32_t was = MODE == SLOT_HAND ? 0u : pr[r];
             pr[r] = 0;
-            if ((uint32_t)r * THREADS + tid < c) {
+            if (r < own) {
                 const uint32_t slot = slot_of(r, was);
                 const uint32_t a = ctr_swizzle<IPT>(slot & ~3u);
                 const uint32_t k8 = slot << 3;  // (shifts take it modulo 32)
                 const uint32_t old = atomicAdd(reinterpret_cast<uint32_t*>(ctr + a), __funnelshift_l(0u, 1u, k8));
                 const uint32_t rank = __funnelshift_r(old, 0u, k8) & 0xFFu;
                 pr[r] = (a | (slot & 3u)) + (rank << 16);
-                rmax = max(rmax, rank);
                 rsum += rank;
                 nmulti += rank == 1u ? 1u : 0u;
             }
+            seen |= pr[r];
         }
-        return !__syncthreads_or(rmax >= SLOT_MAX || rsum > meet * IPT);
+        static_assert(SLOT_MAX == 16, "a rank of 16 or more sets a bit from the 20th on");
+        return !__syncthreads_or((seen >> 20) != 0 || rsum > meet * IPT);
     };
     bool even = false;
     if constexpr (MODE != SLOT_REFINE) {
@@ -441,17 +451,16 @@ __device__ SlotPath block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refi
         // and, in the high half, of the slots with several keys (each counted
         // by the thread whose key came second)
         uint32_t v = nmulti << 16;
-        unsigned char* own = ctr + (size_t)tid * IPT * 4;
         auto quad = [&](int j) {
-            return reinterpret_cast<uint4*>(ctr + ctr_swizzle<IPT>((uint32_t)(own - ctr) + (uint32_t)j * 16));
+            return reinterpret_cast<uint4*>(ctr + ctr_swizzle<IPT>(tid * IPT * 4 + (uint32_t)j * 16));
         };
 #pragma unroll
         for (int j = 0; j < IPT / 4; ++j) {
             const uint4 q = *quad(j);
-            v += (q.x * 0x01010101u) >> 24;
-            v += (q.y * 0x01010101u) >> 24;
-            v += (q.z * 0x01010101u) >> 24;
-            v += (q.w * 0x01010101u) >> 24;
+            v = __dp4a(q.x, 0x01010101u, v);
+            v = __dp4a(q.y, 0x01010101u, v);
+            v = __dp4a(q.z, 0x01010101u, v);
+            v = __dp4a(q.w, 0x01010101u, v);
         }
         uint32_t inc = v;
 #pragma unroll
@@ -489,7 +498,7 @@ __device__ SlotPath block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refi
         // 4. deal the keys into their places, and list the slots of several
 #pragma unroll
         for (int r = 0; r < IPT; ++r) {
-            if ((uint32_t)r * THREADS + tid < c) {
+            if (r < own) {
                 const uint32_t w = *reinterpret_cast<const uint32_t*>(ctr + (pr[r] & 0xFFFCu));
                 const uint32_t rank = pr[r] >> 16;
                 s[(w >> 18) + (((w << 6) >> ((pr[r] & 3u) * 6u)) & 63u) + rank] = key[r];
@@ -533,7 +542,14 @@ __device__ SlotPath block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refi
         }
         __syncthreads();
         // 6. every key is in its final place
-        for (uint32_t p = tid; p < c; p += THREADS) store(p, s[p]);
+        if constexpr (sizeof(K) == 8) {
+            // (unrolled in full, its registers would push out the next keys)
+            for (uint32_t p = tid; p < c; p += THREADS) store(p, s[p]);
+        } else {
+#pragma unroll
+            for (int r = 0; r < IPT; ++r)
+                if (r < own) store((uint32_t)r * THREADS + tid, s[(uint32_t)r * THREADS + tid]);
+        }
     } else if constexpr (MODE != SLOT_HAND) {
         // uneven spread: bitonic leaves + merge path on the same keys
 #pragma unroll
