@@ -64,7 +64,7 @@ static int launch_leaf_class(DevCtx& C, int cls, const LeafItem<K>* items, uint3
         case 1: return launch_leaf_block<K, OutCodec, 128, 8>(C, items, n, out, uneven, n_uneven, st);
         case 2: return launch_leaf_block<K, OutCodec, 256, 8>(C, items, n, out, uneven, n_uneven, st);
         case 3: return launch_leaf_block<K, OutCodec, 256, 16>(C, items, n, out, uneven, n_uneven, st);
-        case 4: return launch_leaf_block<K, OutCodec, 288, 16>(C, items, n, out, uneven, n_uneven, st);
+        case 4: return launch_leaf_block<K, OutCodec, 384, 12>(C, items, n, out, uneven, n_uneven, st);
         case 5: return launch_leaf_block<K, OutCodec, 320, 16>(C, items, n, out, uneven, n_uneven, st);
         case 6: return launch_leaf_block<K, OutCodec, 384, 16>(C, items, n, out, uneven, n_uneven, st);
         case 7: return launch_leaf_block<K, OutCodec, 512, 16>(C, items, n, out, uneven, n_uneven, st);

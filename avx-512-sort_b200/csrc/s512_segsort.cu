@@ -5,7 +5,7 @@
 // data[offsets[s], offsets[s+1])).  The reference sorts such a batch with a
 // loop of SmallSort16V / Sort calls (sort512perf.cpp:612-709 timeSmall).
 // Here: one classification kernel, one persistent launch for the warp-sized
-// segments and one per block size class (1K..16K keys) that has segments,
+// segments and one per block size class (512..16K keys) that has segments,
 // and the partition levels for the few longer segments, all on one stream.
 #include <chrono>
 #include <cstdio>
@@ -20,7 +20,7 @@ namespace s512 {
 // ---------------------------------------------------------------------------
 // The autotuner's search space: the largest block class used (segments above
 // it run the partition levels).  Shape i uses classes 0..kSegShapeTop[i].
-static const int kSegShapeTop[] = {1, 2, 3, 4};
+static const int kSegShapeTop[] = {2, 3, 4, 5};
 constexpr int kNumSegShapes = 4;
 constexpr int kDefaultSegShape = 3;  // blocks of up to 16384 keys
 
@@ -149,13 +149,14 @@ static int launch_classes(DevCtx& C, int shape, Codec io, const SegLists& L, con
         constexpr bool wide = sizeof(typename Codec::Key) == 8;
         int rc;
         switch (c) {
-            case 0: rc = launch_block_class<Codec, 128, 8>(C, io, items, d_n, n, st, prepare_only); break;
-            case 1: rc = launch_block_class<Codec, 256, 8>(C, io, items, d_n, n, st, prepare_only); break;
-            case 2:
+            case 0: rc = launch_block_class<Codec, 64, 8>(C, io, items, d_n, n, st, prepare_only); break;
+            case 1: rc = launch_block_class<Codec, 128, 8>(C, io, items, d_n, n, st, prepare_only); break;
+            case 2: rc = launch_block_class<Codec, 256, 8>(C, io, items, d_n, n, st, prepare_only); break;
+            case 3:
                 rc = wide ? launch_block_class<Codec, 512, 8>(C, io, items, d_n, n, st, prepare_only)
                           : launch_block_class<Codec, 256, 16>(C, io, items, d_n, n, st, prepare_only);
                 break;
-            case 3:
+            case 4:
                 rc = wide ? launch_block_class<Codec, 1024, 8>(C, io, items, d_n, n, st, prepare_only)
                           : launch_block_class<Codec, 512, 16>(C, io, items, d_n, n, st, prepare_only);
                 break;

@@ -23,9 +23,11 @@ struct SegItem {
     uint32_t pad_;
 };
 
-// Block classes: class c holds segments of up to 1024 << c keys.
-constexpr int SEG_NCLASS = 5;
-__host__ __device__ constexpr uint32_t seg_class_cap(int c) { return 1024u << c; }
+// Block classes: class c holds segments of up to 512 << c keys.  (A block of
+// two warps for 257..512 keys: the 1024-key class took 170 us for those and
+// its own of 200k lognormal int32 segments, the two take 61 + 80 us.)
+constexpr int SEG_NCLASS = 6;
+__host__ __device__ constexpr uint32_t seg_class_cap(int c) { return 512u << c; }
 
 struct SegCtl {
     uint32_t n_warp, n_big;
@@ -92,30 +94,56 @@ __global__ void segsort_classify_kernel(const size_t* __restrict__ offsets, size
     }
 }
 
+// A warp's segment of up to 32 * IPT keys at `off`: keys go straight to
+// registers (a network sorts whatever lane they start in), and from there
+// through shared memory to coalesced stores.
+template <int IPT, typename Codec>
+__device__ __forceinline__ void warp_sort_segment(const Codec& io, uint64_t off, uint32_t count,
+                                                  typename Codec::Key* sw) {
+    using K = typename Codec::Key;
+    const unsigned lane = lane_id();
+    K x[IPT];
+#pragma unroll
+    for (int r = 0; r < IPT; ++r) {
+        const uint32_t i = r * 32 + lane;
+        x[r] = i < count ? io.load(off + i) : KeyMax<K>::value;
+    }
+    warp_bitonic_sort<K, IPT>(x);
+    if constexpr (IPT == 1) {
+        if (lane < count) io.store(off + lane, x[0]);
+    } else {
+#pragma unroll
+        for (int r = 0; r < IPT; ++r) sw[pidx(lane * IPT + r)] = x[r];
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < IPT; ++r) {
+            const uint32_t i = r * 32 + lane;
+            if (i < count) io.store(off + i, sw[pidx(i)]);
+        }
+        __syncwarp();
+    }
+}
+
 // Warp segments: one warp per segment (8 warps per block), in place on the
-// caller's layout.
+// caller's layout.  Bound by issue slots: a network of 256 keys takes 288
+// compare steps a lane, one of 128 takes 112, of 64 42, of 32 15, so each
+// segment takes the smallest that holds it (200k lognormal segments, of which
+// 128k are this short: 136 -> 91 us for int32; 50k of doubles: 85 ->
+// 58 us).
 template <typename Codec>
 __global__ void __launch_bounds__(256) segsort_warp_kernel(Codec io, const SegItem* __restrict__ items,
                                                            const SegCtl* __restrict__ ctl) {
     using K = typename Codec::Key;
     __shared__ K stage[8][WARP_REGION];
     const uint32_t nitems = ctl->n_warp;
-    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    const unsigned warp = threadIdx.x >> 5;
     K* sw = stage[warp];
     for (uint32_t w = blockIdx.x * 8 + warp; w < nitems; w += gridDim.x * 8) {
         const SegItem item = items[w];
-        for (uint32_t i = lane; i < (uint32_t)WARP_SEG_MAX; i += 32)
-            sw[pidx(i)] = i < item.count ? io.load(item.off + i) : KeyMax<K>::value;
-        __syncwarp();
-        K x[CHUNK_IPT];
-#pragma unroll
-        for (int r = 0; r < CHUNK_IPT; ++r) x[r] = sw[pidx(lane * CHUNK_IPT + r)];
-        warp_bitonic_sort<K, CHUNK_IPT>(x);
-#pragma unroll
-        for (int r = 0; r < CHUNK_IPT; ++r) sw[pidx(lane * CHUNK_IPT + r)] = x[r];
-        __syncwarp();
-        for (uint32_t i = lane; i < item.count; i += 32) io.store(item.off + i, sw[pidx(i)]);
-        __syncwarp();
+        if (item.count <= 32) warp_sort_segment<1>(io, item.off, item.count, sw);
+        else if (item.count <= 64) warp_sort_segment<2>(io, item.off, item.count, sw);
+        else if (item.count <= 128) warp_sort_segment<4>(io, item.off, item.count, sw);
+        else warp_sort_segment<8>(io, item.off, item.count, sw);
     }
 }
 

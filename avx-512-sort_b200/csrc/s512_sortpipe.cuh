@@ -1414,8 +1414,10 @@ __global__ void __launch_bounds__(256) leaf_warp_kernel(const LeafItem<K>* __res
     }
 }
 
-// Blocks per SM that the leaf kernel's register budget is sized for (the
-// 384-thread class fits three, with its keys' shared memory unpadded).
+// Blocks per SM that the leaf kernel's register budget is sized for.  (The
+// 4608-key class, which holds most buckets of a large sort, has 12 keys per
+// thread: 36 warps an SM instead of 27 with 288 threads of 16, 1.07 -> 1.03 ms
+// of 2^28 doubles.)
 __host__ __device__ constexpr int leaf_min_blocks(int threads) {
     return (threads == 288 || threads == 320 || threads == 384) ? 3 : 1024 / threads;
 }
@@ -1461,7 +1463,7 @@ __global__ void __launch_bounds__(THREADS, leaf_min_blocks(THREADS))
 // host has seen them, and one size of block sorts all classes.  For levels of
 // few keys, where a read-back and a launch per class cost more than blocks
 // that fit their buckets save (2^20 int32: eight leaf launches and their gaps
-// 45 us, this one MEAS_L us).  The host launches what it leaves: larger
+// 45 us, this one 9 us).  The host launches what it leaves: larger
 // buckets, and those found uneven.
 constexpr int ANY_THREADS = 512;
 constexpr int ANY_CLASSES = 8;  // leaf classes 0..7
