@@ -31,6 +31,7 @@ __device__ __forceinline__ uint32_t pidx(uint32_t e) { return e + (e >> 3); }
 // are filled with the maximum here.  All threads of the block must call it.
 template <typename K, int THREADS, int EPT>
 __device__ void block_merge_sort(K* s, uint32_t c) {
+    static_assert(CHUNK % EPT == 0, "a thread's outputs lie in one pair of runs");
     constexpr int NW = THREADS / 32;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     const uint32_t nch = (c + CHUNK - 1) / CHUNK;

@@ -25,7 +25,7 @@ template <> struct PartShapeOne<uint64_t> { static constexpr int THREADS = 512, 
 
 // Slot sort of a class's buckets, then those it found uneven (the second launch reads the count on the device and exits at once
 // when there are none).
-template <typename K, typename OutCodec, int THREADS, int EPT>
+template <typename K, typename OutCodec, int THREADS, int EPT, int UTHREADS = THREADS, int UEPT = EPT>
 static int launch_leaf_block(DevCtx& C, const LeafItem<K>* items, uint32_t n, OutCodec out, LeafItem<K>* uneven,
                              uint32_t* n_uneven, cudaStream_t st) {
     {
@@ -37,11 +37,13 @@ static int launch_leaf_block(DevCtx& C, const LeafItem<K>* items, uint32_t n, Ou
         S512_LAUNCH_CHECK();
     }
     {
-        auto fn = leaf_uneven_kernel<K, OutCodec, THREADS, EPT>;
-        const size_t smem = leaf_uneven_smem<K, OutCodec, THREADS, EPT>();
+        // (the block sort's merges want a power of two of keys per thread)
+        static_assert(UTHREADS * UEPT >= THREADS * EPT, "a bucket of the class fits");
+        auto fn = leaf_uneven_kernel<K, OutCodec, UTHREADS, UEPT>;
+        const size_t smem = leaf_uneven_smem<K, OutCodec, UTHREADS, UEPT>();
         int grid = 0;
-        S512_CUDA_TRY(launch_persistent(C, fn, THREADS, smem, st, (int)n, &grid));
-        fn<<<grid, THREADS, smem, st>>>(uneven, n_uneven, out);
+        S512_CUDA_TRY(launch_persistent(C, fn, UTHREADS, smem, st, (int)n, &grid));
+        fn<<<grid, UTHREADS, smem, st>>>(uneven, n_uneven, out);
         S512_LAUNCH_CHECK();
     }
     return S512_OK;
@@ -64,7 +66,7 @@ static int launch_leaf_class(DevCtx& C, int cls, const LeafItem<K>* items, uint3
         case 1: return launch_leaf_block<K, OutCodec, 128, 8>(C, items, n, out, uneven, n_uneven, st);
         case 2: return launch_leaf_block<K, OutCodec, 256, 8>(C, items, n, out, uneven, n_uneven, st);
         case 3: return launch_leaf_block<K, OutCodec, 256, 16>(C, items, n, out, uneven, n_uneven, st);
-        case 4: return launch_leaf_block<K, OutCodec, 384, 12>(C, items, n, out, uneven, n_uneven, st);
+        case 4: return launch_leaf_block<K, OutCodec, 384, 12, 288, 16>(C, items, n, out, uneven, n_uneven, st);
         case 5: return launch_leaf_block<K, OutCodec, 320, 16>(C, items, n, out, uneven, n_uneven, st);
         case 6: return launch_leaf_block<K, OutCodec, 384, 16>(C, items, n, out, uneven, n_uneven, st);
         case 7: return launch_leaf_block<K, OutCodec, 512, 16>(C, items, n, out, uneven, n_uneven, st);

@@ -92,3 +92,24 @@ def test_segments_of_every_spread(s512, cuda, dt):
     word = pack(keys0, vals0)
     want = torch.cat([torch.sort(word[off[i]:off[i + 1]]).values for i in range(len(parts))])
     assert torch.equal(pack(k, v), want)
+
+
+@pytest.mark.parametrize("n", [4300003, 6000011, 9000001, 14000029])
+def test_uneven_leaves_of_large_arrays(s512, cuda, n):
+    """Levels large enough for a launch per leaf class, with buckets that the
+    slot counts turn away: values that repeat some 18 times, crowded pairs."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    for t0 in (torch.randint(0, n // 18, (n,), dtype=torch.int32, device="cuda", generator=g) * 97,
+               torch.randint(0, n // 18, (n,), dtype=torch.int64, device="cuda", generator=g) << 33,
+               torch.randn(n, dtype=torch.float64, device="cuda", generator=g).mul_(1e4).round_()):
+        t = t0.clone()
+        s512.sort(t)
+        assert torch.equal(t, torch.sort(t0).values)
+    k0 = torch.randint(0, n // 60, (n,), dtype=torch.int32, device="cuda", generator=g) * 9973
+    v0 = torch.arange(n, dtype=torch.int32, device="cuda")
+    k, v = k0.clone(), v0.clone()
+    s512.sort_kv(k, v)
+    want = torch.sort((k0.to(torch.int64) << 32) | v0.to(torch.int64)).values
+    assert torch.equal((k.to(torch.int64) << 32) | v.to(torch.int64), want)
