@@ -105,13 +105,13 @@ static int sort_one_leaf(DevCtx& C, InCodec in, OutCodec out, uint32_t n, cudaSt
         return S512_OK;
     }
     switch (class_of(sizeof(K), n)) {
-        case 1: return launch_small_block<InCodec, OutCodec, 128, 8>(C, in, out, n, st);
-        case 2: return launch_small_block<InCodec, OutCodec, 256, 8>(C, in, out, n, st);
-        case 3: return launch_small_block<InCodec, OutCodec, 512, 8>(C, in, out, n, st);
+        case 1: return launch_small_block<InCodec, OutCodec, 256, 4>(C, in, out, n, st);
+        case 2: return launch_small_block<InCodec, OutCodec, 512, 4>(C, in, out, n, st);
+        case 3: return launch_small_block<InCodec, OutCodec, 1024, 4>(C, in, out, n, st);
         case 4:
         case 5:
         case 6:
-        case 7: return launch_small_block<InCodec, OutCodec, 512, 16>(C, in, out, n, st);
+        case 7: return launch_small_block<InCodec, OutCodec, 1024, 8>(C, in, out, n, st);
         default: return launch_small_block<InCodec, OutCodec, 1024, 16>(C, in, out, n, st);
     }
 }
@@ -185,16 +185,14 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
     if (!samples || !splits || !counts || (fit && !lsets)) return S512_ERR_ALLOC;
 
     const int t0 = tm.mark();
-    init_level_kernel<<<nsegs, NB, 0, st>>>(ctl, counts, L.whole ? L.segs : nullptr, L.first);
-    S512_LAUNCH_CHECK();
     const uint64_t seed = config().seed + 0x9E3779B97F4A7C15ull * (uint64_t)(level + 1);
     {
         // enough blocks per segment to fill the chip (a fed level reads the
         // caller's host arrays where they are)
         uint32_t parts = 2368u / nsegs;
-        parts = parts < 1 ? 1u : parts > SAMPLE_N / 256 ? SAMPLE_N / 256 : parts;
-        sample_kernel<InCodec><<<nsegs * parts, 256, 0, st>>>(feed ? L.in.rebased(feed->mapped) : L.in, L.segs, parts,
-                                                              samples, seed, KB);
+        parts = parts < 1 ? 1u : parts > SAMPLE_N / NB ? SAMPLE_N / NB : parts;
+        sample_kernel<InCodec><<<nsegs * parts, NB, 0, st>>>(feed ? L.in.rebased(feed->mapped) : L.in, L.segs, parts,
+                                                             samples, seed, KB, ctl, counts, L.whole ? 1 : 0, L.first);
         S512_LAUNCH_CHECK();
         auto fn = split_kernel<K>;
         S512_CUDA_TRY(C.prepare((const void*)fn, split_smem<K>()));
@@ -202,7 +200,7 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
                                                               UserOut::PAIRS ? 1 : 0);
         S512_LAUNCH_CHECK();
     }
-    S.kernel_launches += 3;
+    S.kernel_launches += 2;
     int tfit0 = -1;
     if (fit) {
         // the model is fitted to the same sorted sample; the split set above
@@ -295,11 +293,12 @@ static int run_level(DevCtx& C, Level<K, InCodec>& L, int level, UserOut uout, s
         // (a bucket per block at most, as far as the host can tell)
         S512_CUDA_TRY(launch_persistent(C, fn, ANY_THREADS, smem, st, (int)std::min<uint64_t>(nsegs * (uint64_t)NB, 1u << 20),
                                         &grid));
-        fn<<<grid, ANY_THREADS, smem, st>>>(LeafLists<K>{items[0], item_cap}, ctl, uout, any_uneven);
+        fn<<<grid, ANY_THREADS, smem, st>>>(LeafLists<K>{items[0], item_cap}, ctl, uout, any_uneven, host_ctl);
         S512_LAUNCH_CHECK();
         S.kernel_launches += 1;
+    } else {
+        S512_CUDA_TRY(cudaMemcpyAsync(host_ctl, ctl, sizeof(LevelCtl), cudaMemcpyDeviceToHost, st));
     }
-    S512_CUDA_TRY(cudaMemcpyAsync(host_ctl, ctl, sizeof(LevelCtl), cudaMemcpyDeviceToHost, st));
     S512_CUDA_TRY(cudaStreamSynchronize(st));
     bool leaves_done = blind && !host_ctl->err;
 

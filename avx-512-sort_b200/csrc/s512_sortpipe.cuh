@@ -194,6 +194,7 @@ struct LevelCtl {
     uint32_t model_imb_bits;  // largest sample imbalance of a trained model (float bits)
     uint32_t n_uneven[NCLASS];  // leaves handed from the slot sort to the block sort
     uint32_t never_set;       // testing: a flag nothing writes (the injected wait)
+    uint32_t blocks_done;     // leaf_any_kernel: blocks that have ended
     double bucket_sq;         // sum of squared non-empty bucket sizes this level
 };
 
@@ -508,30 +509,27 @@ __device__ bool make_direct(const K (&key)[IPT], uint32_t m, uint64_t count, int
     return true;
 }
 
-// Start of a level (one block per segment): its control block and fill
-// counters zeroed and, for a level that is one whole array, its segment
-// written (one launch instead of a copy and two fills).
-static __global__ void __launch_bounds__(NB) init_level_kernel(LevelCtl* ctl, uint64_t* counts, SegDesc* seg,
-                                                               SegDesc whole) {
-    counts[(size_t)blockIdx.x * NB + threadIdx.x] = 0;
+// Start of a level: keys sampled from every segment, `parts` blocks per
+// segment (random reads are bound by how many one SM can have outstanding, so
+// they are spread over the chip: 16384 reads by one block take 13 us to 33 us,
+// by 64 blocks 2.2 us).  The level's control block and fill counters are zeroed
+// on the way, and the segment of a level that is one `whole` array is written
+// (as launches of their own these cost a small level 4 us).
+template <typename Codec>
+__global__ void __launch_bounds__(NB) sample_kernel(Codec in, SegDesc* __restrict__ segs, uint32_t parts,
+                                                    typename Codec::Key* __restrict__ samples, uint64_t seed,
+                                                    int key_bytes, LevelCtl* ctl, uint64_t* counts, int whole,
+                                                    SegDesc first) {
+    const uint32_t s = blockIdx.x / parts, part = blockIdx.x % parts;
+    if (part == 0) counts[(size_t)s * NB + threadIdx.x] = 0;
     if (blockIdx.x == 0) {
         for (uint32_t i = threadIdx.x; i < sizeof(LevelCtl) / 4; i += NB) reinterpret_cast<uint32_t*>(ctl)[i] = 0;
-        if (seg && threadIdx.x == 0) *seg = whole;
+        if (whole && threadIdx.x == 0) segs[0] = first;
     }
-}
-
-// Keys sampled from every segment, `parts` blocks per segment: random reads
-// are bound by how many one SM can have outstanding, so they are spread over
-// the chip (16384 reads by one block take 13 us to 33 us, by 64 blocks 2.2 us).
-template <typename Codec>
-__global__ void __launch_bounds__(256) sample_kernel(Codec in, const SegDesc* __restrict__ segs, uint32_t parts,
-                                                     typename Codec::Key* __restrict__ samples, uint64_t seed,
-                                                     int key_bytes) {
-    const uint32_t s = blockIdx.x / parts, part = blockIdx.x % parts;
-    const uint64_t in_off = segs[s].in_off, count = segs[s].count;
+    const uint64_t in_off = whole ? first.in_off : segs[s].in_off, count = whole ? first.count : segs[s].count;
     const uint32_t m = sample_size(target_buckets(key_bytes, count));
 #pragma unroll 4
-    for (uint32_t i = part * 256 + threadIdx.x; i < m; i += parts * 256)
+    for (uint32_t i = part * NB + threadIdx.x; i < m; i += parts * NB)
         samples[(size_t)s * SAMPLE_N + i] =
             in.load(in_off + __umul64hi(mix64(seed ^ ((uint64_t)s << 32) ^ (uint64_t)i), count));
 }
@@ -1460,7 +1458,9 @@ __global__ void __launch_bounds__(THREADS, leaf_min_blocks(THREADS))
 
 // Every bucket of up to ANY_CAP keys of a level, and its copies, in one launch
 // that reads the counts on the device: it is queued behind the plan before the
-// host has seen them, and one size of block sorts all classes.  For levels of
+// host has seen them, and one size of block sorts all classes.  Its last block
+// writes the control block to the host's page-locked copy (a copy of its own
+// behind it: 6 us).  For levels of
 // few keys, where a read-back and a launch per class cost more than blocks
 // that fit their buckets save (2^20 int32: eight leaf launches and their gaps
 // 45 us, this one 9 us).  The host launches what it leaves: larger
@@ -1476,13 +1476,14 @@ struct LeafLists {
 };
 template <typename K, typename OutCodec>
 __global__ void __launch_bounds__(ANY_THREADS, 2) leaf_any_kernel(LeafLists<K> lists, LevelCtl* ctl, OutCodec out,
-                                                                  LeafItem<K>* uneven) {
+                                                                  LeafItem<K>* uneven, LevelCtl* host_ctl) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ SlotRed<K> red;
-    if (ctl->err) return;
+    __shared__ uint32_t last;
     uint32_t total = ctl->n_items[CLS_COPY];
 #pragma unroll
     for (int c = 0; c < ANY_CLASSES; ++c) total += ctl->n_items[c];
+    if (ctl->err) total = 0;  // (the host redoes the level, or reports the error)
     for (uint32_t it = blockIdx.x; it < total; it += gridDim.x) {
         uint32_t i = it;
         int c = ANY_CLASSES - 1;  // the largest first, the copies last
@@ -1512,6 +1513,15 @@ __global__ void __launch_bounds__(ANY_THREADS, 2) leaf_any_kernel(LeafLists<K> l
             sort(std::integral_constant<int, 8>{});
         }
         __syncthreads();  // (the two sizes lay out shared memory differently)
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (last) {
+        __threadfence();
+        for (uint32_t i = threadIdx.x; i < sizeof(LevelCtl) / 4; i += ANY_THREADS)
+            reinterpret_cast<volatile uint32_t*>(host_ctl)[i] = reinterpret_cast<volatile uint32_t*>(ctl)[i];
     }
 }
 
