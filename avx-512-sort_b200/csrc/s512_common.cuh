@@ -186,6 +186,12 @@ __device__ __forceinline__ uint64_t shfl_xor<uint64_t>(uint64_t v, int mask) {
     return ((uint64_t)hi << 32) | lo;
 }
 
+// the value of lane `src`
+template <typename T>
+__device__ __forceinline__ T shfl_from(T v, int src) {
+    return __shfl_sync(0xFFFFFFFFu, v, src);
+}
+
 template <typename T>
 __device__ __forceinline__ T kmin(T a, T b) { return a < b ? a : b; }
 template <typename T>

@@ -210,7 +210,7 @@ template <typename K>
 struct alignas(16) BigSlot {
     K lo;
     uint32_t mul;   // (the slot's count until its bounds are known)
-    uint32_t aux;   // first place | shift << 16 | direct << 22 | all equal << 23
+    uint32_t aux;   // first place | shift << 16 | direct << 22 | all equal << 23 | one value << 24
 };
 
 // Fine slots for a bucket whose values crowd: every key's slot of 4*c, rising
@@ -219,7 +219,8 @@ struct alignas(16) BigSlot {
 // fine slots per key, by their place between the slot's own lowest and highest
 // key where it holds many (a cluster, a hot key's values: exact bounds, found
 // by a warp from the dealt keys; equal keys by their rank, so that any number
-// of them fits), by their place in the slot where it holds few.
+// of them fits, also between a few other keys), by their place in the slot
+// where it holds few.
 // Leaves the counters zeroed, a barrier behind.
 template <typename K, int THREADS, int IPT>
 __device__ __forceinline__ void refine_slots(const K (&key)[IPT], uint32_t c, K lo, K range, uint32_t (&fine)[IPT],
@@ -318,12 +319,26 @@ __device__ __forceinline__ void refine_slots(const K (&key)[IPT], uint32_t c, K 
             mx = kmax(mx, shfl_xor(mx, d));
         }
         const SlotMap<K> g = make_slot_map_fast<K>(mn, mx - mn, 4 * n);
+        // mostly one value (a quarter of 32 of the keys)?  Then it takes the
+        // fine slots, and the others, if few, the first and the last one
+        const K x = s[at + lane * n / 32], one = shfl_from(x, 16);
+        bool alone = false;
+        if (mn != mx && __popc(__ballot_sync(0xFFFFFFFFu, x == one)) >= 8) {
+            uint32_t below = 0, above = 0;
+            for (uint32_t i = lane; i < n; i += 32) {
+                below += s[at + i] < one ? 1u : 0u;
+                above += one < s[at + i] ? 1u : 0u;
+            }
+            below = __reduce_add_sync(0xFFFFFFFFu, below);
+            above = __reduce_add_sync(0xFFFFFFFFu, above);
+            alone = below <= SLOT_MAX && above <= SLOT_MAX;
+        }
         __syncwarp();
         if (lane == 0) {
             BigSlot<K> b;
-            b.lo = mn;
-            b.mul = g.mul;
-            b.aux = at | (g.sh << 16) | (g.direct << 22) | (mn == mx ? 1u << 23 : 0u);
+            b.lo = alone ? one : mn;
+            b.mul = alone ? n : g.mul;
+            b.aux = at | (g.sh << 16) | (g.direct << 22) | (mn == mx ? 1u << 23 : 0u) | (alone ? 1u << 24 : 0u);
             big[id] = b;
         }
     }
@@ -337,7 +352,13 @@ __device__ __forceinline__ void refine_slots(const K (&key)[IPT], uint32_t c, K 
                 const BigSlot<K> b = big[(w >> 14) & 0x3FFu];
                 first = b.aux & 0xFFFFu;
                 const uint32_t d = (uint32_t)((key[r] - b.lo) >> ((b.aux >> 16) & 63u));
-                sub = (b.aux >> 23) ? 4u * (w & 0x3FFFu) : (b.aux >> 22) ? d : __umulhi(d, b.mul);
+                const uint32_t by_rank = 4u * (w & 0x3FFFu);
+                if (b.aux >> 24)
+                    sub = key[r] < b.lo ? 0u
+                          : b.lo < key[r] ? 4u * b.mul - 1u
+                                          : min(max(by_rank, 1u), 4u * b.mul - 2u);
+                else
+                    sub = (b.aux >> 23) ? by_rank : (b.aux >> 22) ? d : __umulhi(d, b.mul);
             } else {
                 first = w & 0x3FFFu;
                 const uint32_t d = (uint32_t)((key[r] - lo) >> f.sh);

@@ -39,6 +39,12 @@ def _inputs(n, dtype, seed):
     yield "outlier", t
     yield "cluster", torch.where(full > 0, full >> (bits - 16), full)
     yield "ascending", torch.sort(full).values
+    for share in (3, 20):  # some values repeat, among spread ones, and one has a few close neighbours
+        t = full.clone()
+        hot = full[:8][torch.randint(0, 8, (n,), device="cuda", generator=g)]
+        t = torch.where(rnd(0, share) == 0, hot, t)
+        t[:12] = hot[0] + torch.arange(-6, 6, dtype=dtype, device="cuda")
+        yield f"hot{share}", t
     yield "equal", torch.full((n,), -7, dtype=dtype, device="cuda")
     if dtype == torch.int64:
         for hi in (1, 2, 4095, 4096, 4097):  # distinct high words
