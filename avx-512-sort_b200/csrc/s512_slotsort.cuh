@@ -43,7 +43,7 @@ constexpr uint32_t SLOT_MEET = 3;   // a thread's keys may meet this many earlie
 // Monotone map from a key in [lo, hi] to a slot in [0, nslots): the offset
 // x - lo is cut to its 32 leading significant bits (shift sh), then either
 // used as the slot itself (direct, when the cut range is below nslots) or
-// scaled by mul / 2^32 with mul = floor(nslots * 2^32 / (range + 1)), which
+// scaled by mul / 2^32 with mul just below nslots * 2^32 / (range + 1), which
 // keeps the largest offset below nslots.
 template <typename K>
 struct SlotMap {
@@ -57,26 +57,11 @@ struct SlotMap {
     }
 };
 
+// The slot map of [lo, lo + range].  The quotient is taken in float, rounded
+// down far enough that the largest offset stays below nslots (a 64-bit
+// division costs as much as seven keys of work).
 template <typename K>
-__device__ __forceinline__ SlotMap<K> make_slot_map(K lo, K hi, uint32_t nslots) {
-    SlotMap<K> f;
-    f.lo = lo;
-    const K range = hi - lo;
-    int nb;
-    if constexpr (sizeof(K) == 8) nb = 64 - __clzll((long long)range);
-    else nb = 32 - __clz((int)range);
-    f.sh = nb > 32 ? (uint32_t)(nb - 32) : 0u;
-    const uint32_t dr = (uint32_t)(range >> f.sh);
-    f.direct = dr < nslots ? 1u : 0u;
-    f.mul = f.direct ? 0u : (uint32_t)(((uint64_t)nslots << 32) / ((uint64_t)dr + 1));
-    return f;
-}
-
-// The slot map of a bucket: make_slot_map with the quotient taken in float,
-// rounded down far enough that the largest offset stays below nslots (the
-// 64-bit division of make_slot_map costs as much as seven keys of work).
-template <typename K>
-__device__ __forceinline__ SlotMap<K> make_slot_map_fast(K lo, K range, uint32_t nslots) {
+__device__ __forceinline__ SlotMap<K> make_slot_map(K lo, K range, uint32_t nslots) {
     SlotMap<K> f;
     f.lo = lo;
     int nb;
@@ -240,7 +225,7 @@ __device__ __forceinline__ void refine_slots(const K (&key)[IPT], uint32_t c, K 
     zero();
     __syncthreads();
     // coarse counts; a key's rank in its slot
-    const SlotMap<K> f = make_slot_map_fast<K>(lo, range, S);
+    const SlotMap<K> f = make_slot_map<K>(lo, range, S);
 #pragma unroll
     for (int r = 0; r < IPT; ++r) {
         if ((uint32_t)r * THREADS + tid < c) {
@@ -318,7 +303,7 @@ __device__ __forceinline__ void refine_slots(const K (&key)[IPT], uint32_t c, K 
             mn = kmin(mn, shfl_xor(mn, d));
             mx = kmax(mx, shfl_xor(mx, d));
         }
-        const SlotMap<K> g = make_slot_map_fast<K>(mn, mx - mn, 4 * n);
+        const SlotMap<K> g = make_slot_map<K>(mn, mx - mn, 4 * n);
         // mostly one value (a quarter of 32 of the keys)?  Then it takes the
         // fine slots, and the others, if few, the first and the last one
         const K x = s[at + lane * n / 32], one = shfl_from(x, 16);
@@ -457,7 +442,7 @@ __device__ SlotPath block_slot_sort(K (&key)[IPT], uint32_t c, Store store, Refi
     };
     bool even = false;
     if constexpr (MODE != SLOT_REFINE) {
-        const SlotMap<K> f = make_slot_map_fast<K>(lo, range, NSLOTS);
+        const SlotMap<K> f = make_slot_map<K>(lo, range, NSLOTS);
         even = count(SLOT_MEET, [&](int r, uint32_t) { return f(key[r]); });
     }
     if constexpr (MODE != SLOT_HAND) {

@@ -7,15 +7,16 @@
 // networks.  This file keeps that method and widens each step for a GPU:
 //
 //   * a pivot becomes up to 255 splitters drawn from a random sample of the
-//     segment (sorted on the device), so one partition pass splits a segment
-//     into up to 256 buckets instead of 2;
+//     segment, so one partition pass splits a segment into up to 256 buckets
+//     instead of 2; they lie between value slots where the sample is spread
+//     finely enough over those, else on keys of the sorted sample;
 //   * splitter values that repeat in the sample get an equality bucket (keys
 //     equal to that value need no further sorting), which removes the
 //     reference's quadratic behaviour on few-distinct and sorted inputs;
 //   * the partition pass is out of place and "one sweep": every tile of keys
-//     computes its bucket histogram, reserves its share of each bucket's
-//     output region with one atomic add per bucket, then scatters its keys
-//     through shared memory so global writes are coalesced.  Bucket b of a
+//     gathers its keys by bucket in shared memory, reserves its share of each
+//     bucket's output region with one atomic add per bucket, then writes each
+//     bucket's keys there.  Bucket b of a
 //     segment is written into a region whose capacity comes from the sample
 //     (a 6-sigma bound); a bucket that outgrows it is reported and the level
 //     is redone with exact counts;
@@ -288,7 +289,7 @@ __device__ void make_splitters(Smp smp, uint32_t m, uint64_t count, int nb, Spli
     }
     __syncthreads();
     // splitter lookup table over [sample min, sample max]
-    const SlotMap<K> f = make_slot_map_fast<K>(smp(0), smp(m - 1) - smp(0), (uint32_t)SPLIT_SLOTS);
+    const SlotMap<K> f = make_slot_map<K>(smp(0), smp(m - 1) - smp(0), (uint32_t)SPLIT_SLOTS);
     if (t < NB) w.sk[t] = t < (int)K_u ? f(w.uniq[t]) : 0xFFFFFFFFu;
     if (t == 0) {
         out->slot_map = f;
@@ -385,7 +386,7 @@ __device__ bool make_direct(const K (&key)[IPT], uint32_t m, uint64_t count, int
     for (int j = 0; j < PER / 4; ++j) *quad(j) = make_uint4(0u, 0u, 0u, 0u);
     K lo, range;
     block_bounds<K, THREADS, IPT>(key, m, red, lo, range);
-    const SlotMap<K> f = make_slot_map_fast<K>(lo, range, (uint32_t)DIRECT_SLOTS);
+    const SlotMap<K> f = make_slot_map<K>(lo, range, (uint32_t)DIRECT_SLOTS);
     if (f.direct) return false;  // fewer values than slots
     DirectMap<K> dm;
     dm.lo = lo;
@@ -468,7 +469,7 @@ __device__ bool make_direct(const K (&key)[IPT], uint32_t m, uint64_t count, int
     const bool stands_out = __syncthreads_or((float)cl > 1.6f * share);
     const bool linear = !stands_out && (float)d.sumsq / share - (float)m <= 1.4f * (float)nb + 6.0f;
     if (linear) {
-        dm.mul = make_slot_map_fast<K>(lo, range, (uint32_t)nb).mul;
+        dm.mul = make_slot_map<K>(lo, range, (uint32_t)nb).mul;
     } else {
         uint32_t pack[PER / 4];
 #pragma unroll
@@ -747,9 +748,10 @@ constexpr size_t learned_model_bytes() { return offsetof(LearnedSet<K>, region_o
 // at the same time, lie on different banks.
 __host__ __device__ constexpr int bin_cap(int tile) { return (tile * 5 / 2 / NB) | 1; }
 // A segment's tiles use the bins where that makes an average bin half full at
-// most, and where places in its regions fit 32 bits.
+// most, and where places in its regions (region_bound: 2.01 times its keys)
+// fit 32 bits.
 __host__ __device__ constexpr bool use_bins(int tile, uint32_t nbuckets, uint64_t seg_count) {
-    return (uint32_t)tile * 2 <= nbuckets * (uint32_t)bin_cap(tile) && seg_count < (1ull << 31);
+    return (uint32_t)tile * 2 <= nbuckets * (uint32_t)bin_cap(tile) && seg_count <= 2000000000ull;
 }
 
 template <typename K, int THREADS, int IPT>
@@ -1525,17 +1527,23 @@ __global__ void __launch_bounds__(ANY_THREADS, 2) leaf_any_kernel(LeafLists<K> l
     }
 }
 
-// The buckets the slot sort found uneven.  Of key/value pairs (see
-// block_slot_sort on `refine`): bitonic leaves + merge path; of other keys:
-// refined slots, and that where they are uneven too.
+// Which leaves that came out uneven are dealt a second time before the block
+// sort.  Not key/value pairs (see block_slot_sort on `refine`), nor the leaves
+// of 32-bit arrays: they are uneven because values repeat, several to a coarse
+// slot (2^27 Zipf int32: 3.09 ms a sort with the second dealing, 2.84 without).
+template <typename K, typename OutCodec>
+constexpr bool leaf_refines() { return !OutCodec::PAIRS && sizeof(K) == 8; }
+
+// The buckets the slot sort found uneven: refined slots where leaf_refines, else
+// (and where those are uneven too) bitonic leaves + merge path.
 template <typename K, typename OutCodec, int THREADS, int EPT>
-__global__ void __launch_bounds__(THREADS, OutCodec::PAIRS || 1024 / THREADS < 2 ? 1024 / THREADS : 2)
+__global__ void __launch_bounds__(THREADS, !leaf_refines<K, OutCodec>() || 1024 / THREADS < 2 ? 1024 / THREADS : 2)
     leaf_uneven_kernel(const LeafItem<K>* __restrict__ items, const uint32_t* n_items, OutCodec out) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t nitems = *n_items;
     for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x) {
         const LeafItem<K> item = items[it];
-        if constexpr (OutCodec::PAIRS) {
+        if constexpr (!leaf_refines<K, OutCodec>()) {
             K* s = reinterpret_cast<K*>(smem_raw);
             for (uint32_t i = threadIdx.x; i < item.count; i += THREADS) s[pidx(i)] = item.src[i];
             block_merge_sort<K, THREADS, EPT>(s, item.count);
@@ -1557,7 +1565,7 @@ __global__ void __launch_bounds__(THREADS, OutCodec::PAIRS || 1024 / THREADS < 2
 template <typename K, typename OutCodec, int THREADS, int EPT>
 constexpr size_t leaf_uneven_smem() {
     using SM = SlotSmem<K, THREADS, EPT>;
-    return OutCodec::PAIRS ? SM::padded_bytes : SM::bytes;
+    return leaf_refines<K, OutCodec>() ? SM::bytes : SM::padded_bytes;
 }
 
 // Copy equality buckets (and single keys) to their final place.

@@ -50,7 +50,7 @@ enum {
     S512_OK = 0,
     S512_ERR_ARG = 1,         /* bad argument (null pointer with n > 0, left > right, ...) */
     S512_ERR_ALLOC = 2,       /* device or pinned allocation failed */
-    S512_ERR_TIMEOUT = 3,     /* a bounded device-side wait gave up (look-back spin, bulk copy) */
+    S512_ERR_TIMEOUT = 3,     /* a bounded device-side wait gave up */
     S512_ERR_CUDA = 4,        /* a CUDA runtime call failed; see s512_last_error_string() */
     S512_ERR_INTERNAL = 5,    /* an internal capacity check failed */
     S512_ERR_UNSUPPORTED = 6  /* no usable sm_100 device */
